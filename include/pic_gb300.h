@@ -110,7 +110,8 @@ typedef struct pic_grid {
  * (j-tile x k-row) planes staged in shared memory by bulk asynchronous copies
  * while the CTA marches along i, for grids with no_xy >= 16. AUTO picks
  * STREAM for float32 grids with no_xy >= 64 and no_xy^2 * kpitch >= 1e8 cells,
- * FLAT otherwise; planes_per_item 0 gives about 12 work items per SM,
+ * FLAT otherwise, and segments of small float32 grids run resident
+ * (pic_segment_resident); planes_per_item 0 gives about 12 work items per SM,
  * consumer_warps 0 gives 13, tile_rows 0 about three k-vectors a consumer
  * thread, stages 0 as many as shared memory holds. */
 #define PIC_VARIANT_AUTO 0
@@ -142,6 +143,24 @@ int pic_device_info(int32_t *sm_count, int64_t *total_bytes, int32_t *cc_major, 
  * A workspace of the fixed part alone (ABI 5's size) is still accepted: the
  * deposition then runs without the binned form. */
 int pic_step_workspace_bytes(const pic_grid *g, int64_t *bytes);
+
+/* Bytes of the workspace with which segments of this grid (pic_run_segment,
+ * pic_graph_create, the gradient passes) run as the library prefers: the
+ * step workspace and, for a float32 grid whose fields fit the SMs' registers
+ * and shared memory (up to about a million cells), the resident step's part -- the
+ * deposition pairs and track lists of 256 steps, the packets its blocks
+ * exchange and their tally partials (20 to 200 MB). Allocated and passed as
+ * the step workspace is; a workspace without that part is accepted and those
+ * segments then run one launch a step. */
+int pic_segment_workspace_bytes(const pic_grid *g, int64_t *bytes);
+
+/* 1 if segments of this grid run resident with such a workspace: its blocks
+ * keep the fields on the chip for up to 256 steps a launch. That is the
+ * library's choice for float32 grids of up to about a million cells with
+ * variant AUTO, steps_per_launch 0, a deposit_variant other than TRACKS and
+ * cutoff_voxels < 31.5 (segments of at least 4 steps, 65536 tracks a step at
+ * most); else 0. A segment of a few launches gains nothing from a CUDA graph. */
+int pic_segment_resident(const pic_grid *g, int32_t *resident);
 
 /* Reads (and with reset != 0 clears) the status word a kernel sets in the
  * workspace when a bounded wait gave up: 0 = ok, > 0 = the wait that

@@ -83,6 +83,8 @@ EXPORTS = {
          ctypes.POINTER(ctypes.c_int32)],
     ),
     "pic_step_workspace_bytes": (ctypes.c_int, [ctypes.POINTER(PicGrid), ctypes.POINTER(ctypes.c_int64)]),
+    "pic_segment_workspace_bytes": (ctypes.c_int, [ctypes.POINTER(PicGrid), ctypes.POINTER(ctypes.c_int64)]),
+    "pic_segment_resident": (ctypes.c_int, [ctypes.POINTER(PicGrid), ctypes.POINTER(ctypes.c_int32)]),
     "pic_workspace_status": (
         ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.POINTER(ctypes.c_int32)]
     ),

@@ -32,7 +32,7 @@ import numpy as np
 
 from . import _native as N
 from .config import SimulationConfig
-from .engine import make_grid, nvtx_range
+from .engine import make_grid, nvtx_range, runs_resident
 from .feeder import TrackFeeder
 from .pulses import TrackSampler, build_track_schedule
 from .state import Diagnostics, collection_efficiency
@@ -577,7 +577,7 @@ def run_batched_b200(
         need = 0
         for g in grids:  # one workspace for every solo grid: the largest any of them needs
             swb = ctypes.c_int64()
-            N.check(lib.pic_step_workspace_bytes(ctypes.byref(g), ctypes.byref(swb)), "pic_step_workspace_bytes")
+            N.check(lib.pic_segment_workspace_bytes(ctypes.byref(g), ctypes.byref(swb)), "pic_segment_workspace_bytes")
             need = max(need, int(swb.value))
         solo_ws = torch.zeros(need, dtype=torch.uint8, device=dev)
 
@@ -587,9 +587,9 @@ def run_batched_b200(
         """Grid c's global steps [c0, c1) with the single-grid kernels, on its
         slices: state of step s in buffer s & 1, deposition pairs in buffer
         s & 1 (the batched step clears the other one every step, as
-        pic_run_segment expects), tallies at row tally_off + s. The chunk's
-        launches are captured into one CUDA graph and replayed (small grids
-        are launch-bound)."""
+        pic_run_segment expects), tallies at row tally_off + s. A grid that
+        does not run resident has its chunk's launches captured into one CUDA
+        graph and replayed (small grids are launch-bound)."""
         fo, do2 = field_off[c] * es, 2 * dens_off[c] * es
         off = np.ascontiguousarray(offsets[c][c0 : c1 + 1])
         args = (ctypes.byref(grids[c]), pos[0].data_ptr() + fo, neg[0].data_ptr() + fo, pos[1].data_ptr() + fo,
@@ -597,6 +597,9 @@ def run_batched_b200(
                 ys_dev.data_ptr() + 8 * track_base[c], off.ctypes.data, dens[0].data_ptr() + do2,
                 dens[1].data_ptr() + do2, c0 & 1, counts.data_ptr() + 4 * counts_off[c],
                 tally.data_ptr() + 32 * (tally_off[c] + c0), solo_ws.data_ptr(), solo_ws.numel(), st)
+        if runs_resident(grids[c]):
+            N.check(lib.pic_run_segment(*args), "pic_run_segment")
+            return
         h = ctypes.c_void_p()
         N.check(lib.pic_graph_create(*args, ctypes.byref(h)), "pic_graph_create")
         solo_graphs.append(h.value)

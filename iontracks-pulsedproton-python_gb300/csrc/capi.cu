@@ -204,6 +204,24 @@ static int check_fields(const void *a, const void *b, const void *c, const void 
     return PIC_OK;
 }
 
+// The caller's pair buffers after a segment that deposited into the workspace,
+// as the per-step forms leave them: buffer `last` holds the last step's pairs
+// if it deposited (null: it did not), the other one is zero for the step after
+// the segment.
+static int leave_pairs(const pic_grid *g, void *const dens[2], int last, const void *last_pairs, cudaStream_t st) {
+    const int64_t pb = dens_pitch(g->no_xy) * 2 * g->no_xy * (g->dtype == PIC_F64 ? 8 : 4);
+    if (last_pairs) {
+        cudaError_t e = cudaMemcpyAsync(dens[last], last_pairs, (size_t)pb, cudaMemcpyDeviceToDevice, st);
+        if (e != cudaSuccess) return set_cuda_error("cudaMemcpyAsync(deposition pairs)", e);
+    }
+    cudaError_t e = cudaMemsetAsync(dens[last ^ 1], 0, (size_t)pb, st);
+    return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaMemsetAsync(deposition pairs)", e);
+}
+
+static cudaError_t clear_bin_counts(const pic_grid *g, void *ws, cudaStream_t st) {
+    return cudaMemsetAsync(static_cast<char *>(ws) + kWorkspaceBytes, 0, (size_t)bin_count_bytes(g->no_xy), st);
+}
+
 static int run_loop(const pic_grid *g, void *pos0, void *neg0, void *pos1, void *neg1, int64_t parity,
                     int64_t n_steps, const double *xs, const double *ys, const int64_t *off, void *dens0,
                     void *dens1, int64_t dens_parity, uint32_t *counts, double *tally, void *ws,
@@ -226,9 +244,27 @@ static int run_loop(const pic_grid *g, void *pos0, void *neg0, void *pos1, void 
         }
         return PIC_OK;
     }
+    ResPlan plan;
+    if (resident_steps_eligible(g, ws, ws_bytes, off, n_steps, &plan)) {
+        const void *last_pairs = nullptr;
+        int bi = (int)(parity & 1);
+        for (int64_t s0 = 0; s0 < n_steps;) {
+            const int64_t s1 = next_resident_group(off, s0, n_steps);
+            const int bo = (int)((parity + s1) & 1);
+            int rc = resident_steps(g, plan, pos[bi], neg[bi], pos[bo], neg[bo], xs, ys, off, s0, s1, counts,
+                                    tally + 4 * s0, nullptr, 0, &last_pairs, ws, st);
+            if (rc) return rc;
+            bi = bo;
+            s0 = s1;
+        }
+        return leave_pairs(g, dens, (int)((dens_parity + n_steps - 1) & 1), last_pairs, st);
+    }
     int64_t most = 0;
     for (int64_t s = 0; s < n_steps; ++s) most = std::max(most, off[s + 1] - off[s]);
     if (most > 0 && most <= kBinTracks && deposit_binned(g, ws, ws_bytes, most)) {
+        // (another grid may have left its own lists where this one's counts are)
+        cudaError_t e = clear_bin_counts(g, ws, st);
+        if (e != cudaSuccess) return set_cuda_error("cudaMemsetAsync(tile counts)", e);
         // the binned deposition of up to kBinSteps steps (kBinTracks tracks)
         // at a time into the workspace's pair buffers, then those steps
         const void *dp[kBinSpan];
@@ -247,17 +283,7 @@ static int run_loop(const pic_grid *g, void *pos0, void *neg0, void *pos1, void 
             if (s1 == n_steps) last_pairs = dp[s1 - 1 - s0];
             s0 = s1;
         }
-        // The caller's pair buffers, as the per-step forms leave them: the
-        // last step's pairs if it deposited, and a zero buffer for the step
-        // after the segment.
-        const int64_t pb = dens_pitch(g->no_xy) * 2 * g->no_xy * (g->dtype == PIC_F64 ? 8 : 4);
-        const int last = (int)((dens_parity + n_steps - 1) & 1);
-        if (last_pairs) {
-            cudaError_t e = cudaMemcpyAsync(dens[last], last_pairs, (size_t)pb, cudaMemcpyDeviceToDevice, st);
-            if (e != cudaSuccess) return set_cuda_error("cudaMemcpyAsync(deposition pairs)", e);
-        }
-        cudaError_t e = cudaMemsetAsync(dens[last ^ 1], 0, (size_t)pb, st);
-        return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaMemsetAsync(deposition pairs)", e);
+        return leave_pairs(g, dens, (int)((dens_parity + n_steps - 1) & 1), last_pairs, st);
     }
     for (int64_t s = 0; s < n_steps; ++s) {
         const int bi = (int)((parity + s) & 1), bo = bi ^ 1;
@@ -381,6 +407,24 @@ int pic_step_workspace_bytes(const pic_grid *g, int64_t *bytes) {
     if (rc) return rc;
     if (!bytes) return set_error(PIC_E_INVALID, "bytes is null");
     *bytes = kWorkspaceBytes + dep_bin_bytes(g);
+    return PIC_OK;
+}
+
+int pic_segment_workspace_bytes(const pic_grid *g, int64_t *bytes) {
+    int rc = check_grid(g);
+    if (rc) return rc;
+    if (!bytes) return set_error(PIC_E_INVALID, "bytes is null");
+    ResPlan plan;
+    *bytes = resident_plan(g, &plan) ? resident_space(g, plan).end : kWorkspaceBytes + dep_bin_bytes(g);
+    return PIC_OK;
+}
+
+int pic_segment_resident(const pic_grid *g, int32_t *resident) {
+    int rc = check_grid(g);
+    if (rc) return rc;
+    if (!resident) return set_error(PIC_E_INVALID, "resident is null");
+    ResPlan plan;
+    *resident = resident_wanted(g) && bin_eligible(g) && resident_plan(g, &plan) ? 1 : 0;
     return PIC_OK;
 }
 

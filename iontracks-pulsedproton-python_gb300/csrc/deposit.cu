@@ -204,6 +204,32 @@ int launch_deposit_steps(const pic_grid *g, const double *xs, const double *ys, 
                                : launch_binned_steps<float>(g, xs, ys, off, s0, s1, counts, ws, targets, dens, st);
 }
 
+int launch_deposit_slots(const pic_grid *g, const double *xs, const double *ys, const int64_t *off, int64_t s0,
+                         int64_t s1, uint32_t *hist, void *ws, const ResSpace &r, void *dens, int64_t dens_stride,
+                         int16_t *slot, cudaStream_t st) {
+    BinSlotsSteps<float> S{};
+    int k = 0;
+    for (int64_t s = s0; s < s1; ++s) {
+        slot[s - s0] = -1;
+        if (off[s + 1] == off[s]) continue;
+        if (k == kResSteps) return set_error(PIC_E_INVALID, "more than kResSteps depositing steps in one launch");
+        S.off[k] = (int32_t)(off[s] - off[s0]);
+        slot[s - s0] = (int16_t)k++;
+    }
+    if (k == 0) return PIC_OK;
+    S.count = k;
+    S.tracks = off[s1] - off[s0];
+    S.off[k] = (int32_t)S.tracks;
+    if (S.tracks > kBinTracks) return set_error(PIC_E_INVALID, "more than kBinTracks tracks in one launch");
+    DepBins<float> bins = dep_bins<float>(ws, g->no_xy);
+    char *w = static_cast<char *>(ws);
+    bins.count = reinterpret_cast<int *>(w + r.counts);
+    bins.list = reinterpret_cast<int *>(w + r.lists);
+    S.base = grid_slot<float>(g, bins, 0, xs + off[s0], ys + off[s0], 0, S.tracks, dens, hist, 0);
+    S.dens_stride = dens_stride;
+    return binned_launches<float>(S, bins.scratch, k * bins.tiles, st);
+}
+
 int64_t next_deposit_group(const int64_t *off, int64_t s0, int64_t n_steps, int64_t *n_dep) {
     int64_t s1 = s0, nd = 0;
     while (s1 < n_steps && s1 - s0 < kBinSpan) {

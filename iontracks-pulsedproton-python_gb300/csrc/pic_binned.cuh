@@ -71,6 +71,39 @@ struct BinSlotsValue {
     }
 };
 
+// The steps of one resident launch over one grid: up to kResSteps slots that
+// differ in their tracks and in where their pairs and lists go.
+template <typename T>
+struct BinSlotsSteps {
+    BinSlot<T> base;      // slot 0's
+    int64_t dens_stride;  // pairs from one slot's to the next's
+    int count;
+    int64_t tracks;
+    int32_t off[kResSteps + 1];  // slot k: launch tracks [off[k], off[k + 1])
+    __device__ __forceinline__ BinSlot<T> operator[](int k) const {
+        const int64_t tiles = (int64_t)base.tps * base.tps;
+        BinSlot<T> s = base;
+        s.first = off[k];
+        s.last = off[k + 1];
+        s.xs += s.first;
+        s.ys += s.first;
+        s.dens += k * dens_stride;
+        s.count += k * tiles;
+        s.list += k * tiles * kBinCap;
+        s.block0 = (int32_t)(k * tiles);
+        return s;
+    }
+    __device__ __forceinline__ int of_track(int64_t t) const {
+        int lo = 0, hi = count - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (off[mid] <= t) lo = mid; else hi = mid - 1;
+        }
+        return lo;
+    }
+    __device__ __forceinline__ int of_block(int64_t b) const { return (int)(b / ((int64_t)base.tps * base.tps)); }
+};
+
 // Slots in device memory (a batched global step's grids, written by the
 // step's preparation kernel): binary searches over first and block0.
 template <typename T>

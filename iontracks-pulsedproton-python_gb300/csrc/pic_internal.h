@@ -207,6 +207,71 @@ constexpr int kBinMaxSlots = 1024;
 int64_t batched_deposit_bytes(int32_t n_cfgs, int32_t total_tiles, int64_t max_tracks, int64_t dens_bytes,
                               int32_t dtype);
 
+// The resident step (resident.cu): how a float32 grid is divided over blocks
+// that keep it on the chip for up to kResSteps steps of one launch. ti x tj
+// columns and tkv k-vectors a block (nti x ntj x ntk of them), a patch of
+// columns a thread (gi x gj patches, `threads` of them), `aux` threads beside
+// the chain, `packets` a block publishes per step.
+constexpr int kResSteps = 256;
+constexpr int kResMinSteps = 4;  // shorter segments step by step (two launches a step)
+constexpr int64_t kResMaxNoXy = 1024;
+struct ResPlan {
+    int patch, nti, ntj, ntk, ti, tj, tkv, gi, gj, blocks, threads, aux, smem, packets;
+};
+// The division of this grid; false when it does not fit the chip.
+bool resident_plan(const pic_grid *g, ResPlan *out);
+// `steps` steps from pos_in/neg_in. keep_stride 0: the last step's state into
+// pos_out/neg_out (which may be the input for an even number of steps); > 0:
+// step s's state at pos_out/neg_out + s * keep_stride. slot[s]: the pairs of
+// step s at dens + slot[s] * dens_stride, -1: none. tally null: none wanted.
+int launch_resident(const pic_grid *g, const ResPlan &p, const void *pos_in, const void *neg_in, void *pos_out,
+                    void *neg_out, const void *dens, int64_t dens_stride, const int16_t *slot, int steps,
+                    int64_t keep_stride, double *tally, void *packets, void *partials, int *status, cudaStream_t st);
+// The resident step's part of the step workspace, behind the binned
+// deposition's: the tile counts of kResSteps slots and the packets (one clear
+// before a launch), the launch's tally partials and, where the binned
+// deposition can run, the slots' track lists and pairs.
+struct ResSpace {
+    int64_t counts, packets, partials, lists, dens, end;  // byte offsets from the workspace's start
+};
+inline ResSpace resident_space(const pic_grid *g, const ResPlan &p) {
+    const int64_t tiles = bin_tiles_per_side(g->no_xy) * bin_tiles_per_side(g->no_xy);
+    const bool bins = bin_eligible(g);
+    ResSpace r;
+    r.counts = kWorkspaceBytes + dep_bin_bytes(g);
+    r.packets = r.counts + (bins ? bin_align(kResSteps * tiles * 4) : 0);
+    r.partials = r.packets + bin_align(2LL * p.blocks * p.packets * 16);
+    r.lists = r.partials + bin_align((int64_t)kResSteps * p.blocks * p.aux);  // 32 bytes a warp
+    r.dens = r.lists + (bins ? kResSteps * tiles * kBinCap * 4 : 0);
+    r.end = r.dens + (bins ? kResSteps * bin_dens_bytes(g->no_xy, 4) : 0);
+    return r;
+}
+// Whether the grid leaves the choice of kernels to the library.
+inline bool resident_wanted(const pic_grid *g) {
+    return g->variant == PIC_VARIANT_AUTO && g->steps_per_launch == 0 && g->deposit_variant != PIC_DEPOSIT_TRACKS;
+}
+// Whether a segment of these steps runs resident: the library's own choice of
+// kernels (no variant, steps per launch or per-track deposition asked for), a
+// workspace of pic_step_workspace_bytes, and tracks the binned deposition takes.
+bool resident_steps_eligible(const pic_grid *g, const void *ws, int64_t ws_bytes, const int64_t *off, int64_t n_steps,
+                             ResPlan *plan);
+// The end of the next resident launch's steps from s0 (at most kResSteps of
+// them and kBinTracks tracks).
+int64_t next_resident_group(const int64_t *off, int64_t s0, int64_t n_steps);
+// Deposits and runs steps s0 .. s1 - 1 (a group of next_resident_group) from
+// pos_in/neg_in into pos_out/neg_out. targets: where the pairs go, one slot of
+// target_stride pairs per step with tracks (null: into the workspace).
+// *last_pairs: the last step's pairs (null: no tracks).
+int resident_steps(const pic_grid *g, const ResPlan &plan, const void *pos_in, const void *neg_in, void *pos_out,
+                   void *neg_out, const double *xs, const double *ys, const int64_t *off, int64_t s0, int64_t s1,
+                   uint32_t *counts, double *tally, void *targets, int64_t target_stride, const void **last_pairs,
+                   void *ws, cudaStream_t st);
+// The binned deposition of the steps of one resident launch, a slot per step
+// with tracks; slot[s - s0] receives step s's (-1: none).
+int launch_deposit_slots(const pic_grid *g, const double *xs, const double *ys, const int64_t *off, int64_t s0,
+                         int64_t s1, uint32_t *hist, void *ws, const ResSpace &r, void *dens, int64_t dens_stride,
+                         int16_t *slot, cudaStream_t st);
+
 // Whether the deposition takes the binned form for this grid and workspace:
 // for a segment's steps together (most = the most tracks one of them has),
 // or with most < 0 for one step alone.

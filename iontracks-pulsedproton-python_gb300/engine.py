@@ -65,6 +65,14 @@ def resolve_shape(g: N.PicGrid) -> dict:
     return d
 
 
+def runs_resident(g: N.PicGrid) -> bool:
+    """Whether segments of this descriptor keep the fields on the chip for
+    hundreds of steps a launch (``pic_segment_resident``)."""
+    out = ctypes.c_int32()
+    N.check(N.load().pic_segment_resident(ctypes.byref(g), ctypes.byref(out)), "pic_segment_resident")
+    return bool(out.value)
+
+
 def make_grid(config, dtype: str = "float32", alpha_cm3_s: float | None = None, shape: dict | None = None) -> N.PicGrid:
     """The ``pic_grid`` descriptor of a configuration (any object with the
     reference SimulationConfig's attributes), with optional launch-shape
@@ -138,7 +146,7 @@ class ChamberEngine:
         steps = int(config.total_time_steps) if tally_steps is None else int(tally_steps)
         self.tally = torch.zeros((max(steps, 1), 4), dtype=torch.float64, **kw)
         wsb = ctypes.c_int64()
-        N.check(self.lib.pic_step_workspace_bytes(ctypes.byref(g), ctypes.byref(wsb)), "pic_step_workspace_bytes")
+        N.check(self.lib.pic_segment_workspace_bytes(ctypes.byref(g), ctypes.byref(wsb)), "pic_segment_workspace_bytes")
         self.workspace = torch.zeros(int(wsb.value), dtype=torch.uint8, **kw)
         self.xs = torch.zeros(max(int(max_tracks), 1), dtype=torch.float64, **kw)
         self.ys = torch.zeros(max(int(max_tracks), 1), dtype=torch.float64, **kw)

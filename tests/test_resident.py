@@ -1,0 +1,167 @@
+"""The resident step (csrc/resident.cu): segments of small float32 grids whose
+blocks keep the fields on the chip, against the float64 flat step on the same
+state, tracks and steps.
+
+Tolerance: a float32 step rounds each value about ten times against weights
+that sum to one in absolute value 1.4 at most, so it is off by up to
+10 * 6e-8 * 1.4 < 1e-6 of the peak a step, and the steps' errors add at worst:
+1e-6 * steps, fields and tallies alike (every tally sums values of one sign)."""
+
+import ctypes
+import importlib
+
+import numpy as np
+import pytest
+
+from goldens import make_config, pkg
+
+# no_xy, no_z, voxels of the chamber's grid: one block and many, ragged tiles
+# and k splits, a patch of every shape, the smallest and the largest that run
+# resident, k rows with one and with eight padded elements
+SIZES = [(3, 1), (4, 3), (5, 20), (8, 50), (11, 50), (12, 200), (13, 43), (24, 200), (25, 149), (31, 100), (48, 200),
+         (53, 200), (48, 400), (59, 400), (70, 203), (76, 200)]
+
+
+def _grid(native, n, no_z, wall, dtype, variant):
+    g = native.PicGrid()
+    g.no_xy, g.no_z, g.nze = n, no_z, 2
+    g.nzb = no_z + 4
+    g.kpitch = (g.nzb + 7) // 8 * 8
+    g.mid_xy = n / 2
+    g.scoring_radius_sq = max(1.0, (n / 2 - 3) ** 2)
+    g.p_lat, g.p_zm, g.p_zp = 0.02, 0.52, -0.06
+    g.n_lat, g.n_zm, g.n_zp = 0.03, 0.70, -0.05
+    g.p_cen = 1 - 4 * g.p_lat - g.p_zm - g.p_zp
+    g.n_cen = 1 - 4 * g.n_lat - g.n_zm - g.n_zp
+    g.alpha_dt = 2e-4
+    g.gaussian_factor, g.h2_over_b2, g.cutoff_voxels = 3.0, 0.11, 6.5
+    g.wall, g.dtype, g.variant = wall, dtype, variant
+    return g
+
+
+def _segment(native, g, torch, state, xs, ys, off, parity, graph=False, workspace="pic_segment_workspace_bytes"):
+    lib = native.load()
+    t = torch.float64 if g.dtype == native.PIC_F64 else torch.float32
+    n, kp, steps = g.no_xy, g.kpitch, len(off) - 1
+    f = [torch.zeros((n, n, kp), dtype=t, device="cuda") for _ in range(4)]
+    for q in range(2):
+        f[2 * parity + q][:, :, : g.nzb] = torch.from_numpy(state[q]).to("cuda", t)
+    dens = [torch.zeros((n, 2 * ((n + 3) // 4 * 4)), dtype=t, device="cuda") for _ in range(2)]
+    counts = torch.zeros((n, n), dtype=torch.int32, device="cuda")
+    tally = torch.zeros((steps, 4), dtype=torch.float64, device="cuda")
+    b = ctypes.c_int64()
+    native.check(getattr(lib, workspace)(ctypes.byref(g), ctypes.byref(b)), workspace)
+    ws = torch.zeros(b.value, dtype=torch.uint8, device="cuda")
+    x, y = torch.from_numpy(xs).cuda(), torch.from_numpy(ys).cuda()
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    args = (ctypes.byref(g), f[0].data_ptr(), f[1].data_ptr(), f[2].data_ptr(), f[3].data_ptr(), parity, steps,
+            x.data_ptr(), y.data_ptr(), off.ctypes.data, dens[0].data_ptr(), dens[1].data_ptr(), parity,
+            counts.data_ptr(), tally.data_ptr(), ws.data_ptr(), ws.numel(), st.cuda_stream)
+    if graph:
+        h = ctypes.c_void_p()
+        native.check(lib.pic_graph_create(*args, ctypes.byref(h)), "pic_graph_create")
+        native.check(lib.pic_graph_launch(h, st.cuda_stream), "pic_graph_launch")
+    else:
+        native.check(lib.pic_run_segment(*args), "pic_run_segment")
+    status = ctypes.c_int32()
+    native.check(lib.pic_workspace_status(ws.data_ptr(), 0, st.cuda_stream, ctypes.byref(status)), "status")
+    if graph:
+        native.check(lib.pic_graph_destroy(h), "pic_graph_destroy")
+    assert status.value == 0
+    out = (parity + steps) & 1
+    return (f[2 * out][:, :, : g.nzb].double().cpu().numpy(), f[2 * out + 1][:, :, : g.nzb].double().cpu().numpy(),
+            f[2 * out][:, :, g.nzb :].abs().sum().item() + f[2 * out + 1][:, :, g.nzb :].abs().sum().item(),
+            tally.cpu().numpy(), counts.cpu().numpy(), [d.double().cpu().numpy() for d in dens])
+
+
+def _case(n, no_z, steps, seed, most_tracks):
+    rng = np.random.default_rng(seed)
+    state = [np.zeros((n, n, no_z + 4)) for _ in range(2)]
+    for s in state:  # every column its own, the ring's too
+        s[:, :, 1:-1] = rng.uniform(0.5, 1.5, (n, n, no_z + 2))
+    m = rng.integers(0, most_tracks + 1, steps) * (rng.random(steps) < 0.7)
+    off = np.concatenate([[0], np.cumsum(m)]).astype(np.int64)
+    return state, rng.uniform(0, n, off[-1] + 1), rng.uniform(0, n, off[-1] + 1), off
+
+
+def _compare(native, got, ref, steps):
+    tol = 1e-6 * steps
+    for a, b in zip(got[:2], ref[:2]):
+        assert np.abs(a - b).max() <= tol * np.abs(b).max()
+    assert got[2] == 0.0
+    for q in range(4):
+        peak = np.abs(ref[3][:, q]).max()
+        assert np.abs(got[3][:, q] - ref[3][:, q]).max() <= tol * peak + 1e-30
+    assert np.array_equal(got[4], ref[4])
+    for a, b in zip(got[5], ref[5]):  # the caller's pair buffers, as every segment leaves them
+        assert np.abs(a - b).max() <= 1e-6 * max(1.0, np.abs(b).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("wall", [0, 1])
+@pytest.mark.parametrize("n,no_z", SIZES)
+def test_resident_segment_matches_the_float64_step(n, no_z, wall):
+    import torch
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    steps = 9
+    state, xs, ys, off = _case(n, no_z, steps, 100 * n + no_z + wall, 12)
+    g = _grid(native, n, no_z, wall, native.PIC_F32, 0)
+    resident = ctypes.c_int32()
+    native.check(native.load().pic_segment_resident(ctypes.byref(g), ctypes.byref(resident)), "pic_segment_resident")
+    assert resident.value == 1
+    parity = n & 1
+    before = native.load().pic_kernel_launches()
+    got = _segment(native, g, torch, state, xs, ys, off, parity)
+    assert native.load().pic_kernel_launches() - before <= 4  # binning, tiles, steps, tallies
+    ref = _segment(native, _grid(native, n, no_z, wall, native.PIC_F64, 1), torch, state, xs, ys, off, parity)
+    _compare(native, got, ref, steps)
+    again = _segment(native, g, torch, state, xs, ys, off, parity, graph=True)
+    for a, b in zip(got[:4], again[:4]):  # the same bits, from a replayed graph
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,no_z,steps,tracks", [(10, 50, 600, 3), (24, 100, 300, 20), (31, 60, 12, 30000)])
+def test_resident_segments_of_several_launches(n, no_z, steps, tracks):
+    """More steps than one launch takes, and more tracks than one deposition does."""
+    import torch
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    state, xs, ys, off = _case(n, no_z, steps, n, tracks)
+    for wall in (0, 1):
+        g = _grid(native, n, no_z, wall, native.PIC_F32, 0)
+        g64 = _grid(native, n, no_z, wall, native.PIC_F64, 1)
+        g.gaussian_factor = g64.gaussian_factor = 3.0 / tracks
+        got = _segment(native, g, torch, state, xs, ys, off, 0)
+        ref = _segment(native, g64, torch, state, xs, ys, off, 0)
+        _compare(native, got, ref, steps)
+
+
+def test_what_runs_resident():
+    """The choice follows the descriptor alone: AUTO float32 grids that fit,
+    nothing that asks for a kernel or has truncation boxes beyond 64 cells."""
+    native = importlib.import_module(pkg().__name__ + "._native")
+    lib = native.load()
+
+    def resident(**kw):
+        g = _grid(native, kw.pop("n", 24), kw.pop("no_z", 200), 0, kw.pop("dtype", native.PIC_F32), kw.pop("variant", 0))
+        for k, v in kw.items():
+            setattr(g, k, v)
+        out, seg, step = ctypes.c_int32(), ctypes.c_int64(), ctypes.c_int64()
+        native.check(lib.pic_segment_resident(ctypes.byref(g), ctypes.byref(out)), "pic_segment_resident")
+        native.check(lib.pic_segment_workspace_bytes(ctypes.byref(g), ctypes.byref(seg)), "pic_segment_workspace_bytes")
+        native.check(lib.pic_step_workspace_bytes(ctypes.byref(g), ctypes.byref(step)), "pic_step_workspace_bytes")
+        assert seg.value >= step.value
+        return bool(out.value)
+
+    assert resident()
+    assert resident(deposit_variant=native.PIC_DEPOSIT_BINNED)
+    assert not resident(deposit_variant=native.PIC_DEPOSIT_TRACKS)
+    assert not resident(variant=1) and not resident(steps_per_launch=32) and not resident(dtype=native.PIC_F64)
+    assert not resident(cutoff_voxels=31.5)
+    assert not resident(n=208, no_z=400) and not resident(n=1068, no_z=400)
+    engine = importlib.import_module(pkg().__name__ + ".engine")
+    assert engine.runs_resident(engine.make_grid(make_config("column_10um_r008")))
+    assert not engine.runs_resident(engine.make_grid(make_config("column_10um_r02", track_cutoff_sigmas=None)))
