@@ -337,7 +337,9 @@ int pic_adjoint_forward(const pic_grid *g, void *pos0, void *neg0, void *pos1, v
  * the last, recompute the segment's states from its checkpoint into
  * states_pos/neg (ckpt_every states, state_stride apart; kept densities, no
  * deposition, no tallies), then run the adjoint
- * steps over them backwards. lambda starts at zero in buffer 0 of
+ * steps over them backwards (grids that run resident, adjoint_variant AUTO,
+ * the workspace of pic_segment_workspace_bytes: each in one launch, the
+ * checkpoint itself read as the segment's first state). lambda starts at zero in buffer 0 of
  * (lam_*0, lam_*1) (both zeroed by the caller); lambda_0 ends in buffer
  * n_steps & 1. grad[0..4] receives dR/d(s+, c+, s-, c-, alpha_dt) summed
  * over all steps (each step's terms as pic_adjoint_step's). Workspaces: the

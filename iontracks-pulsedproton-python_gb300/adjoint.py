@@ -54,7 +54,7 @@ import numpy as np
 from . import _native as N
 from .config import lax_wendroff_weights
 from .constants import recombination_alpha
-from .engine import ChamberEngine
+from .engine import ChamberEngine, runs_resident
 from .pulses import TrackSampler, build_track_schedule
 from .state import collection_efficiency
 
@@ -120,8 +120,9 @@ class AdjointRun:
     schedule's state slots (default: as many as the memory limit allows, at
     most one per step). ``shape``: launch shape of the step kernels
     (``{"variant": "flat" | "stream", ..., "adjoint_variant": ...}``);
-    default: the autotuned step shape (as :func:`run_simulation_b200`) and the
-    library's choice of adjoint kernel for the grid.
+    default: for grids that run resident (``engine.runs_resident``) the
+    library's choice, for others the autotuned step shape (as
+    :func:`run_simulation_b200`) and the library's adjoint kernel.
     """
 
     def __init__(self, config, theta=None, checkpoint_every: int = 64, dtype: str = "float32", rng=None,
@@ -206,7 +207,7 @@ class AdjointRun:
         np.cumsum(schedule, out=self.offsets[1:])
         eng = ChamberEngine(cfg, dtype=self.dtype, max_tracks=max(1, n_tracks), tally_steps=max(total, 1),
                             shape=self.shape)
-        if self.shape is None:
+        if self.shape is None and (self.schedule == "binomial" or not runs_resident(eng.grid)):
             from .autotune import tune
 
             tune(eng, quick=True)  # on the fresh (zero) fields: leaves them zero

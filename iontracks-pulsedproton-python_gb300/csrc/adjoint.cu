@@ -42,6 +42,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
 
 #include "pic_adjoint.cuh"
@@ -445,15 +446,20 @@ int launch_adjoint(const pic_grid *g, const void *pos, const void *neg, const vo
     return launch_adjoint_t<float>(g, pos, neg, dens, lp_in, ln_in, lp_out, ln_out, grad, ws, st, accumulate);
 }
 
+double *adjoint_slots(void *ws) { return reinterpret_cast<double *>(static_cast<char *>(ws) + adj_counter_bytes()); }
+
+// Slots of a backward sweep: the flat and the streaming kernel's blocks, and
+// the resident one's (at most one per SM).
+static int64_t adjoint_slot_count(const pic_grid *g) { return std::max<int64_t>(adjoint_blocks(g), sm_count()); }
+
 int adjoint_accumulate_begin(const pic_grid *g, void *ws, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(static_cast<char *>(ws) + adj_counter_bytes(), 0,
-                                    (size_t)(adjoint_blocks(g) * kAdjGrad * 8), st);
+    cudaError_t e = cudaMemsetAsync(adjoint_slots(ws), 0, (size_t)(adjoint_slot_count(g) * kAdjGrad * 8), st);
     return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaMemsetAsync(adjoint slots)", e);
 }
 
 int adjoint_accumulate_end(const pic_grid *g, void *ws, double *grad, cudaStream_t st) {
-    const double *slots = reinterpret_cast<const double *>(static_cast<char *>(ws) + adj_counter_bytes());
-    const int nb = (int)adjoint_blocks(g);
+    const double *slots = adjoint_slots(ws);
+    const int nb = (int)adjoint_slot_count(g);
     if (g->dtype == PIC_F64)
         adjoint_collect_kernel<double, 256><<<1, 256, 0, st>>>(slots, nb, grad);
     else

@@ -602,9 +602,29 @@ int pic_adjoint_forward(const pic_grid *g, void *pos0, void *neg0, void *pos1, v
                                 cudaMemcpyDeviceToDevice, st);
         return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaMemcpyAsync(checkpoint)", e);
     };
+    ResPlan plan;
+    if (ckpt_every >= kResMinSteps && resident_steps_eligible(g, workspace, workspace_bytes, track_offsets, n_steps, &plan)) {
+        // launches up to the next checkpoint, pairs straight into the kept slots
+        const void *last_pairs = nullptr;
+        int64_t d = 0;
+        for (int64_t s0 = 0; s0 < n_steps;) {
+            const int64_t end = std::min(n_steps, (s0 / ckpt_every + 1) * ckpt_every);
+            const int64_t s1 = next_resident_group(track_offsets, s0, end);
+            if ((rc = checkpoint(s0))) return rc;
+            const int b = (int)(s0 & 1), bo = (int)(s1 & 1);
+            if ((rc = resident_steps(g, plan, pos[b], neg[b], pos[bo], neg[bo], xs, ys, track_offsets, s0, s1, counts,
+                                     tally + 4 * s0, D + d * dslot * es, dslot / 2, &last_pairs, workspace, st)))
+                return rc;
+            for (int64_t s = s0; s < s1; ++s) d += track_offsets[s + 1] > track_offsets[s];
+            s0 = s1;
+        }
+        return PIC_OK;
+    }
     int64_t most = 0;
     for (int64_t s = 0; s < n_steps; ++s) most = std::max(most, track_offsets[s + 1] - track_offsets[s]);
     if (most > 0 && most <= kBinTracks && deposit_binned(g, workspace, workspace_bytes, most)) {
+        cudaError_t e = clear_bin_counts(g, workspace, st);
+        if (e != cudaSuccess) return set_cuda_error("cudaMemsetAsync(tile counts)", e);
         // each launch pair deposits up to kBinSteps steps straight into their
         // kept slots
         const void *dp[kBinSpan];
@@ -654,6 +674,39 @@ int pic_adjoint_forward(const pic_grid *g, void *pos0, void *neg0, void *pos1, v
     return PIC_OK;
 }
 
+// One checkpoint segment of L steps backwards on the chip: its states 1 .. L - 1
+// recomputed from the checkpoint (state j at SP/SN + j * stride), then the
+// adjoint steps (adj_plan null: the caller's). slot[j]: the kept pairs of step j
+// (-1: none).
+static int resident_segment_back(const pic_grid *g, const ResPlan &plan, const ResPlan *adj_plan, const char *cp,
+                                 const char *cn, char *SP, char *SN, int64_t stride, int L, const int64_t *slot,
+                                 const char *dens, int64_t dens_stride, void *lp_in, void *ln_in, void *lp_out,
+                                 void *ln_out, void *adj_ws, void *ws, cudaStream_t st) {
+    const ResSpace r = resident_space(g, plan);
+    char *w = static_cast<char *>(ws);
+    int *status = workspace_layout(ws).status;
+    int64_t first = -1;  // the segment's kept slots are consecutive
+    int16_t at[kResSteps];
+    for (int j = 0; j < L; ++j) {
+        if (slot[j] >= 0 && first < 0) first = slot[j];
+        at[j] = slot[j] < 0 ? (int16_t)-1 : (int16_t)(slot[j] - first);
+    }
+    const char *D = first < 0 ? dens : dens + first * dens_stride * 8;
+    auto clear = [&]() {
+        cudaError_t e = cudaMemsetAsync(w + r.packets, 0, (size_t)(r.partials - r.packets), st);
+        return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaMemsetAsync(packets)", e);
+    };
+    int rc = clear();
+    if (rc) return rc;
+    if ((rc = launch_resident(g, plan, cp, cn, SP + 4 * stride, SN + 4 * stride, D, dens_stride, at, L - 1, stride, nullptr,
+                              w + r.packets, w + r.partials, status, st)))
+        return rc;
+    if (!adj_plan) return PIC_OK;
+    if ((rc = clear())) return rc;
+    return launch_resident_adjoint(g, *adj_plan, cp, cn, SP, SN, stride, D, dens_stride, at, L, lp_in, ln_in, lp_out, ln_out,
+                                   adjoint_slots(adj_ws), w + r.packets, status, st);
+}
+
 int pic_adjoint_backward(const pic_grid *g, const void *ckpt_pos, const void *ckpt_neg, int64_t state_stride,
                          int64_t n_steps, int64_t ckpt_every, const int64_t *track_offsets, const void *dens_keep,
                          void *states_pos, void *states_neg, void *lam_pos0, void *lam_neg0, void *lam_pos1,
@@ -695,9 +748,29 @@ int pic_adjoint_backward(const pic_grid *g, const void *ckpt_pos, const void *ck
     int cur = 0;  // lambda_{n_steps} = 0 in buffer 0
     const int64_t n_seg = (n_steps + ckpt_every - 1) / ckpt_every;
     if ((rc = adjoint_accumulate_begin(g, adj_workspace, st))) return rc;
+    // small grids: a launch recomputes a segment's states, another runs its
+    // adjoint steps (resident.cu, adjoint_resident.cu)
+    ResPlan plan, adj_plan;
+    const bool resident = resident_wanted(g) && ckpt_every <= kResSteps && resident_plan(g, &plan) &&
+                          workspace_bytes >= resident_space(g, plan).end;
+    const bool resident_adjoint = resident && g->adjoint_variant == PIC_VARIANT_AUTO && resident_adjoint_plan(g, &adj_plan);
     for (int64_t c = n_seg - 1; c >= 0; --c) {
         const int64_t s0 = c * ckpt_every, s1 = (s0 + ckpt_every < n_steps) ? s0 + ckpt_every : n_steps;
         const int64_t L = s1 - s0;
+        const bool on_chip = resident && L >= kResMinSteps;
+        if (on_chip) {
+            const char *cp = static_cast<const char *>(ckpt_pos) + c * state_stride * es;
+            const char *cn = static_cast<const char *>(ckpt_neg) + c * state_stride * es;
+            const int out = (cur + (int)L) & 1;
+            if ((rc = resident_segment_back(g, plan, resident_adjoint ? &adj_plan : nullptr, cp, cn, SP, SN, state_stride,
+                                            (int)L, &slot[s0], D, dslot / 2, lp[cur], ln[cur], lp[out], ln[out],
+                                            adj_workspace, workspace, st)))
+                return rc;
+            if (resident_adjoint) {
+                cur = out;
+                continue;
+            }
+        }
         cudaError_t e = cudaMemcpyAsync(SP, static_cast<const char *>(ckpt_pos) + c * state_stride * es,
                                         (size_t)(field * es), cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess)
@@ -705,7 +778,7 @@ int pic_adjoint_backward(const pic_grid *g, const void *ckpt_pos, const void *ck
                                 cudaMemcpyDeviceToDevice, st);
         if (e != cudaSuccess) return set_cuda_error("cudaMemcpyAsync(checkpoint)", e);
         // recompute states s0 .. s1-1 of the segment (state j at slot j - s0)
-        for (int64_t j = 0; j + 1 < L; ++j) {
+        for (int64_t j = 0; j + 1 < L && !on_chip; ++j) {
             rc = launch_step(g, SP + j * state_stride * es, SN + j * state_stride * es, SP + (j + 1) * state_stride * es,
                              SN + (j + 1) * state_stride * es, dens_of(s0 + j), nullptr, nullptr, workspace, st);
             if (rc) return rc;

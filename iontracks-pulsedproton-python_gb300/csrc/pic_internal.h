@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
 
 #include <nvtx3/nvToolsExt.h>
@@ -227,6 +228,16 @@ bool resident_plan(const pic_grid *g, ResPlan *out);
 int launch_resident(const pic_grid *g, const ResPlan &p, const void *pos_in, const void *neg_in, void *pos_out,
                     void *neg_out, const void *dens, int64_t dens_stride, const int16_t *slot, int steps,
                     int64_t keep_stride, double *tally, void *packets, void *partials, int *status, cudaStream_t st);
+// The division of this grid for the resident adjoint; false when it does not fit.
+bool resident_adjoint_plan(const pic_grid *g, ResPlan *out);
+// Adjoint steps steps - 1 .. 0 of a checkpoint segment: step 0 from the state
+// pos0/neg0, step j > 0 from pos/neg + j * state_stride; lambda from lp_in/ln_in
+// to lp_out/ln_out (the same buffers for an even number of steps only); the
+// derivative sums join the blocks' slots (adjoint_accumulate_begin).
+int launch_resident_adjoint(const pic_grid *g, const ResPlan &p, const void *pos0, const void *neg0, const void *pos,
+                            const void *neg, int64_t state_stride, const void *dens, int64_t dens_stride,
+                            const int16_t *slot, int steps, const void *lp_in, const void *ln_in, void *lp_out,
+                            void *ln_out, double *slots, void *packets, int *status, cudaStream_t st);
 // The resident step's part of the step workspace, behind the binned
 // deposition's: the tile counts of kResSteps slots and the packets (one clear
 // before a launch), the launch's tally partials and, where the binned
@@ -235,12 +246,15 @@ struct ResSpace {
     int64_t counts, packets, partials, lists, dens, end;  // byte offsets from the workspace's start
 };
 inline ResSpace resident_space(const pic_grid *g, const ResPlan &p) {
+    ResPlan adj;
+    int64_t packets = 2LL * p.blocks * p.packets * 16;
+    if (resident_adjoint_plan(g, &adj)) packets = std::max<int64_t>(packets, 2LL * adj.blocks * adj.packets * 16);
     const int64_t tiles = bin_tiles_per_side(g->no_xy) * bin_tiles_per_side(g->no_xy);
     const bool bins = bin_eligible(g);
     ResSpace r;
     r.counts = kWorkspaceBytes + dep_bin_bytes(g);
     r.packets = r.counts + (bins ? bin_align(kResSteps * tiles * 4) : 0);
-    r.partials = r.packets + bin_align(2LL * p.blocks * p.packets * 16);
+    r.partials = r.packets + bin_align(packets);
     r.lists = r.partials + bin_align((int64_t)kResSteps * p.blocks * p.aux);  // 32 bytes a warp
     r.dens = r.lists + (bins ? kResSteps * tiles * kBinCap * 4 : 0);
     r.end = r.dens + (bins ? kResSteps * bin_dens_bytes(g->no_xy, 4) : 0);
@@ -334,6 +348,7 @@ bool adjoint_stream_eligible(const pic_grid *g);
 int launch_adjoint_stream(const pic_grid *g, const void *pos, const void *neg, const void *dens, const void *lp_in,
                           const void *ln_in, void *lp_out, void *ln_out, double *grad, unsigned int *counter,
                           int *status, double *partials, int64_t max_blocks, cudaStream_t st, bool accumulate);
+double *adjoint_slots(void *ws);  // the blocks' running sums in the adjoint workspace
 int adjoint_accumulate_end(const pic_grid *g, void *ws, double *grad, cudaStream_t st);
 
 // Binomial checkpointing (revolve.cu).

@@ -47,37 +47,26 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <mutex>
 #include <type_traits>
 
-#include "pic_device.cuh"
-#include "pic_flat.cuh"
-#include "pic_internal.h"
-#include "pic_packet.cuh"
+#include "pic_resident.cuh"
 
 namespace pic {
 
 namespace {
 
-struct ResArgs {
+struct ResArgs : ResShape {
     const float *pos_in, *neg_in;
     float *pos_out, *neg_out;
     const float2 *dens;   // pairs of slot q at dens + q * dens_stride
     int64_t dens_stride;
-    uint4 *packets;       // [2][blocks][face_total]
     float2 *partials;     // [steps][blocks][aux warps][4] double-floats
-    int *status;
     int64_t keep_stride;  // > 0: every step's state is stored, step s's at out + s * keep_stride; 0: the last one's
-    int n, kp, c4, nzb, nze, gap_end, reflecting, dp, steps;
-    int nti, ntj, ntk, ti, tj, tkv, gi, gj;
-    int patch_threads, aux_threads;  // the roles of a block's threads, in this order
+    int dp, steps;
     float2 p_lat, p_zm, p_zp, p_cen, n_lat, n_zm, n_zp, n_cen, alpha_dt;  // each twice, for packed arithmetic
     ScoreTest score;
     int16_t slot[kResSteps];  // pair slot of each step, -1: no tracks
 };
-
-__device__ __forceinline__ float4 ld4s(const float *p) { return *reinterpret_cast<const float4 *>(p); }
-__device__ __forceinline__ void st4s(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
 
 // a + b, exactly (Knuth's TwoSum, as in df_add).
 __device__ __forceinline__ DF two_sum(float a, float b) {
@@ -101,46 +90,11 @@ __device__ __forceinline__ DF warp_sum4(const DF (&v)[4], int lane) {
     return s;
 }
 
-// Offsets of a block's six faces in its packet region. A lateral face holds
-// [packet][column][k-vector], three packets an item (i_side or j_side apart);
-// a k face one packet a column.
-struct Faces {
-    int i_side, j_side, im, ip, jm, jp, km, kp, total;
-};
-__host__ __device__ inline Faces res_faces(int ti, int tj, int tkv) {
-    Faces f;
-    f.i_side = tj * tkv;
-    f.j_side = ti * tkv;
-    f.im = 0;
-    f.ip = f.im + 3 * f.i_side;
-    f.jm = f.ip + 3 * f.i_side;
-    f.jp = f.jm + 3 * f.j_side;
-    f.km = f.jp + 3 * f.j_side;
-    f.kp = f.km + ti * tj;
-    f.total = f.kp + ti * tj;
-    return f;
-}
-
-__device__ __forceinline__ void send_item(uint4 *p, int side, float4 P, float4 N, uint32_t tag) {
-    packet_store(p, __float_as_uint(P.x), __float_as_uint(P.y), __float_as_uint(P.z), tag);
-    packet_store(p + side, __float_as_uint(P.w), __float_as_uint(N.x), __float_as_uint(N.y), tag);
-    packet_store(p + 2 * side, __float_as_uint(N.z), __float_as_uint(N.w), 0u, tag);
-}
-
-__device__ __forceinline__ float masked(float x, uint32_t m) { return __uint_as_float(__float_as_uint(x) & m); }
-
 // Shared memory: two buffers of deposition pairs over the block's columns (ring
 // and halo included), two buffers of the threads' tallies, one or two buffers
 // of the cells ([row][column][species][4 + 4 TKV] and 4 floats more, a row and a
 // column more on each side), and the table of what the block trades.
-__host__ __device__ inline int res_cells(int gi, int gj, int RI, int RJ) { return (gi * RI + 2) * (gj * RJ + 2); }
 __host__ __device__ inline int res_pair_floats(int cells) { return (4 * cells + 3) / 4 * 4; }
-// (four floats between two rows of k: the one above the lower row's end, ..,
-// the one below the next row's start; 120 floats a column, so that the lanes
-// of a warp that go on into the next column of 13 or 14 k-vectors also go on
-// through the banks)
-__host__ __device__ constexpr int res_pitch(int tkv_max) { return 4 * tkv_max + 4; }
-
 __host__ __device__ constexpr bool res_small(int ri, int rj) { return ri * rj < 6; }
 template <int RI, int RJ, int TKV, int MAXT, bool MIRROR>
 __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant__ ResArgs a) {
@@ -152,39 +106,18 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
     extern __shared__ __align__(16) float res_smem[];
     __shared__ volatile int s_abort;
     const int tid = threadIdx.x, T = a.patch_threads, lane = tid & 31;
-    const int cta = blockIdx.x;
-    const int bk = cta % a.ntk, bj = (cta / a.ntk) % a.ntj, bi = cta / (a.ntk * a.ntj);
-    const int n = a.n, kp = a.kp, tkv = a.tkv, steps = a.steps;
-    const int i0 = 1 + bi * a.ti, j0 = 1 + bj * a.tj, kv0 = bk * tkv;
-    const int rows = min(a.ti, n - 1 - i0), cols = min(a.tj, n - 1 - j0), kvn = min(tkv, a.c4 - kv0);
     const int W = a.gj * RJ + 2, ROW = W * COL;
+    ResTile<PITCH> tile(a, W);
+    const int cta = tile.cta, bk = tile.bk, i0 = tile.i0, j0 = tile.j0, kv0 = tile.kv0;
+    const int rows = tile.rows, cols = tile.cols, kvn = tile.kvn, n_side = tile.n_side, n_around = tile.n_around;
+    const bool lo_i = tile.lo_i, hi_i = tile.hi_i, lo_j = tile.lo_j, hi_j = tile.hi_j;
+    const int n = a.n, kp = a.kp, tkv = a.tkv, steps = a.steps;
     const int ncell = res_cells(a.gi, a.gj, RI, RJ);
     float2 *pairs = reinterpret_cast<float2 *>(res_smem);  // [2][ncell]
     float *sums = res_smem + res_pair_floats(ncell);       // [2][3][T]
     float *S = sums + 6 * T;
     const int BUF = SMALL ? ncell * COL + 4 : 0;  // floats from one buffer of cells to the other
-    const Faces F = res_faces(a.ti, a.tj, tkv);
-    const bool lo_i = bi > 0, hi_i = bi + 1 < a.nti, lo_j = bj > 0, hi_j = bj + 1 < a.ntj;
-    const bool lo_k = bk > 0, hi_k = bk + 1 < a.ntk;
-    const int64_t region = (int64_t)gridDim.x * F.total;  // packets of one parity of steps
     const bool trades = gridDim.x > 1;  // cells with other blocks
-    auto cell_of = [&](int r, int c) { return ((r + 1) * W + c + 1) * COL + 4; };
-
-    // The columns around the block: the sides i-, i+, j-, j+, then the corners.
-    const int n_side = 2 * cols + 2 * rows, n_around = n_side + 4;
-    auto around = [&](int u, int &r, int &c) {
-        if (u < cols) r = -1, c = u;
-        else if (u < 2 * cols) r = rows, c = u - cols;
-        else if (u < 2 * cols + rows) c = -1, r = u - 2 * cols;
-        else if (u < n_side) c = cols, r = u - 2 * cols - rows;
-        else r = (u - n_side) & 1 ? rows : -1, c = (u - n_side) & 2 ? cols : -1;
-    };
-    // Whether column u of them is a ring column this block keeps (a corner of
-    // the block is one where it is the grid's corner).
-    auto ring_col = [&](int u, int r, int c) {
-        const int i = i0 + r, j = j0 + c;
-        return (i == 0 || i == n - 1) + (j == 0 || j == n - 1) >= (u < n_side ? 1 : 2);
-    };
 
     // ---- load: cells to zero, then the block's values and its surroundings ----
     if (tid == 0) s_abort = 0;
@@ -194,57 +127,22 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
     for (int u = tid; u < n_around * kvn; u += blockDim.x) {
         const int col = u / kvn, v = u - col * kvn;
         int r, c;
-        around(col, r, c);
-        if (col >= n_side && !ring_col(col, r, c)) continue;  // nobody's neighbour
+        tile.around(col, r, c);
+        if (col >= n_side && !tile.ring_col(col, r, c)) continue;  // nobody's neighbour
         const int64_t o = ((int64_t)(i0 + r) * n + (j0 + c)) * kp + 4 * (kv0 + v);
-        float *d = S + cell_of(r, c) + 4 * v;
+        float *d = S + tile.cell_of(r, c) + 4 * v;
         st4s(d, *reinterpret_cast<const float4 *>(a.pos_in + o));
         st4s(d + PITCH, *reinterpret_cast<const float4 *>(a.neg_in + o));
     }
     for (int u = tid; u < rows * cols; u += blockDim.x) {
         const int r = u / cols, c = u - r * cols;
         const int64_t o = ((int64_t)(i0 + r) * n + (j0 + c)) * kp + 4 * kv0;
-        float *d = S + cell_of(r, c);
-        if (lo_k) d[-1] = a.pos_in[o - 1], d[PITCH - 1] = a.neg_in[o - 1];
-        if (hi_k) d[4 * kvn] = a.pos_in[o + 4 * kvn], d[PITCH + 4 * kvn] = a.neg_in[o + 4 * kvn];
+        float *d = S + tile.cell_of(r, c);
+        if (tile.lo_k) d[-1] = a.pos_in[o - 1], d[PITCH - 1] = a.neg_in[o - 1];
+        if (tile.hi_k) d[4 * kvn] = a.pos_in[o + 4 * kvn], d[PITCH + 4 * kvn] = a.neg_in[o + 4 * kvn];
     }
 
-    // What the block trades: lateral item u of trade[] is a cell of the block's
-    // edge, sent, and the cell beyond it, taken in; item h_lat + u the same of
-    // the k faces (one element). x: its packet to send, y: to take, z and w:
-    // the cells from and to (lateral: z both, in units of four floats; w the
-    // distance of its three packets).
-    const int h_im = lo_i ? cols * kvn : 0, h_ip = hi_i ? cols * kvn : 0;
-    const int h_jm = lo_j ? rows * kvn : 0, h_jp = hi_j ? rows * kvn : 0;
-    const int h_lat = h_im + h_ip + h_jm + h_jp;
-    const int h_km = lo_k ? rows * cols : 0, h_k = h_km + (hi_k ? rows * cols : 0);
-    int4 *const trade = reinterpret_cast<int4 *>(S + (SMALL ? 2 : 1) * (ncell * COL + 4));
-    for (int q = tid; q < h_lat; q += blockDim.x) {
-        int u = q, nb, own_face, its_face, r, c, dr = 0, dc = 0, along;
-        if (u < h_im + h_ip) {
-            const bool up = u >= h_im;
-            if (up) u -= h_im;
-            c = along = u / kvn, u -= c * kvn;
-            r = up ? rows - 1 : 0, dr = up ? 1 : -1;
-            nb = dr * a.ntj * a.ntk, own_face = up ? F.ip : F.im, its_face = up ? F.im : F.ip;
-        } else {
-            u -= h_im + h_ip;
-            const bool up = u >= h_jm;
-            if (up) u -= h_jm;
-            r = along = u / kvn, u -= r * kvn;
-            c = up ? cols - 1 : 0, dc = up ? 1 : -1;
-            nb = dc * a.ntk, own_face = up ? F.jp : F.jm, its_face = up ? F.jm : F.jp;
-        }
-        const int o = along * tkv + u;
-        trade[q] = make_int4(cta * F.total + own_face + o, (cta + nb) * F.total + its_face + o,
-                             (cell_of(r, c) / 4 + u) | (cell_of(r + dr, c + dc) / 4 + u) << 16, dr ? F.i_side : F.j_side);
-    }
-    for (int q = tid; q < h_k; q += blockDim.x) {
-        const bool up = q >= h_km;
-        const int u = up ? q - h_km : q, r = u / cols, c = u - r * cols, o = r * a.tj + c, d = cell_of(r, c);
-        trade[h_lat + q] = make_int4(cta * F.total + (up ? F.kp : F.km) + o, (cta + (up ? 1 : -1)) * F.total + (up ? F.km : F.kp) + o,
-                                     d + (up ? 4 * kvn - 1 : 0), d + (up ? 4 * kvn : -1));
-    }
+    tile.table(reinterpret_cast<int4 *>(S + (SMALL ? 2 : 1) * (ncell * COL + 4)));
 
     if (tid >= T) {
         // ---------------- the warps beside the steps' chain ----------------
@@ -320,7 +218,7 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
     asm volatile("" : "+r"(gm0), "+r"(gm1), "+r"(gm2), "+r"(gm3), "+r"(gkm), "+r"(gkp));
     const bool all_valid = k0 >= 1 && k0 + 3 <= a.nzb - 2;
     const int r_last = rows - 1 - rb, c_last = cols - 1 - cb;
-    float *const cell0 = S + cell_of(rb, cb) + 4 * kvt;
+    float *const cell0 = S + tile.cell_of(rb, cb) + 4 * kvt;
     const float2 *const pair0 = pairs + (rb + 1) * W + cb + 1;
     // edges of the patch on a reflecting wall, whose ring mirrors them (the row or
     // column within the patch, -1: none)
@@ -344,80 +242,6 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
             }
         }
 
-    // Sends the block's face cells of the step that gives `tag`.
-    auto give = [&](const float *B, uint32_t tag) {
-        uint4 *const out = a.packets + (tag & 1 ? region : 0);
-#pragma unroll 1
-        for (int u = tid; u < h_lat; u += T) {
-            const int4 e = trade[u];
-            const float *d = B + (e.z & 0xffff) * 4;
-            send_item(out + e.x, e.w, ld4s(d), ld4s(d + PITCH), tag);
-        }
-#pragma unroll 1
-        for (int u = tid; u < h_k; u += T) {
-            const int4 e = trade[h_lat + u];
-            packet_store(out + e.x, __float_as_uint(B[e.z]), __float_as_uint(B[e.z + PITCH]), 0u, tag);
-        }
-    };
-    // Takes in the cells beyond them; false when they did not come. A thread
-    // polls for LAT lateral items and K k items at once, from items u and v on,
-    // every T-th; past the last one it takes that one again (the same values).
-    auto take_some = [&](auto lats, auto ks, const uint4 *in, float *B, uint32_t tag, int u, int v) {
-        constexpr int LAT = decltype(lats)::value, KS = decltype(ks)::value;
-        const uint4 *p[LAT + 1], *pk = nullptr;
-        int side[LAT + 1], d[LAT + 1], dk = 0;
-#pragma unroll
-        for (int x = 0; x < LAT; ++x) {
-            const int4 e = trade[min(u + x * T, h_lat - 1)];
-            p[x] = in + e.y, side[x] = e.w, d[x] = (int)((unsigned)e.z >> 16) * 4;
-        }
-        if (KS) {
-            const int4 e = trade[h_lat + min(v, h_k - 1)];
-            pk = in + e.y, dk = e.w;
-        }
-        uint4 V[LAT + 1][3], K;
-        for (int polls = 0;; ++polls) {
-#pragma unroll
-            for (int x = 0; x < LAT; ++x)
-#pragma unroll
-                for (int y = 0; y < 3; ++y) V[x][y] = packet_load(p[x] + y * side[x]);
-            if (KS) K = packet_load(pk);
-            uint32_t off = KS ? K.w ^ tag : 0u;
-#pragma unroll
-            for (int x = 0; x < LAT; ++x) off |= (V[x][0].w ^ tag) | (V[x][1].w ^ tag) | (V[x][2].w ^ tag);
-            if (off == 0) break;
-            if ((polls & 1023) == 1023 && (polls > kPacketPolls || *reinterpret_cast<volatile int *>(a.status) != 0)) {
-                atomicCAS(a.status, 0, kPacketTimeout);
-                return false;
-            }
-        }
-#pragma unroll
-        for (int x = 0; x < LAT; ++x) {
-            st4s(B + d[x], make_float4(__uint_as_float(V[x][0].x), __uint_as_float(V[x][0].y),
-                                       __uint_as_float(V[x][0].z), __uint_as_float(V[x][1].x)));
-            st4s(B + d[x] + PITCH, make_float4(__uint_as_float(V[x][1].y), __uint_as_float(V[x][1].z),
-                                               __uint_as_float(V[x][2].x), __uint_as_float(V[x][2].y)));
-        }
-        if (KS) {
-            B[dk] = __uint_as_float(K.x);
-            B[dk + PITCH] = __uint_as_float(K.y);
-        }
-        return true;
-    };
-    auto take = [&](float *B, uint32_t tag) {
-        using C0 = std::integral_constant<int, 0>;
-        using C1 = std::integral_constant<int, 1>;
-        using C2 = std::integral_constant<int, 2>;
-        const uint4 *const in = a.packets + (tag & 1 ? region : 0);
-        int u = tid, v = tid, left = h_lat, left_k = h_k;  // the block's items still to take
-        bool ok = true;
-        if (left > 0 && left_k > 0)
-            ok = left > T ? take_some(C2{}, C1{}, in, B, tag, u, v) : take_some(C1{}, C1{}, in, B, tag, u, v),
-            u += 2 * T, v += T, left -= 2 * T, left_k -= T;
-        for (; ok && left > 0; u += 2 * T, left -= 2 * T) ok = take_some(C2{}, C0{}, in, B, tag, u, v);
-        for (; ok && left_k > 0; v += T, left_k -= T) ok = take_some(C0{}, C1{}, in, B, tag, u, v);
-        return ok;
-    };
     // The absorbing ring from the cells of step s into those of step s + 1: its
     // own value and the step's deposition.
     const bool carries = !MIRROR && (!lo_i || !hi_i || !lo_j || !hi_j);
@@ -432,9 +256,9 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
         for (int u = tid; u < n_around * kvn; u += T) {
             const int col = u / kvn, v = u - col * kvn;
             int r, c;
-            around(col, r, c);
-            if (!ring_col(col, r, c)) continue;
-            const int d = cell_of(r, c) + 4 * v;
+            tile.around(col, r, c);
+            if (!tile.ring_col(col, r, c)) continue;
+            const int d = tile.cell_of(r, c) + 4 * v;
             float4 RP = ld4s(from + d), RN = ld4s(from + d + PITCH);
             const float dd = dep ? Dp[(r + 1) * W + c + 1].x : 0.f;
 #pragma unroll
@@ -593,7 +417,7 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
         pair_now = ncell - pair_now;
         if (trades) {
             __syncthreads();  // the block's new cells are in
-            if (send) give(S + now, (uint32_t)(s + 1));
+            if (send) tile.give(S + now, (uint32_t)(s + 1));
         }
         // while the packets are on their way: the tallies (the aux warps sum
         // them during the next step), the wall's ring, the states to keep
@@ -625,7 +449,7 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
                     }
         }
         if (!MIRROR && carries) carry_ring(s);
-        if (trades && send && !take(S + now, (uint32_t)(s + 1))) s_abort = 1;
+        if (trades && send && !tile.take(S + now, (uint32_t)(s + 1))) s_abort = 1;
     }
     __syncthreads();
 }
@@ -648,46 +472,20 @@ __global__ void __launch_bounds__(256) resident_tally_kernel(const float2 *parti
     if ((lane & 7) == 0) tally[4 * (int64_t)s + (lane >> 3)] = df_value(w) * (lane == 0 ? injected_scale : 1.0);
 }
 
-// The patches a thread may own, with the block size their registers allow, and
-// the longest k range of a block.
-struct Patch {
-    int ri, rj, max_threads;
-};
-constexpr Patch kPatches[] = {{1, 1, 640}, {2, 1, 512}, {2, 2, 512}, {3, 2, 448}, {4, 2, 384}};
-constexpr int kPatchCount = sizeof(kPatches) / sizeof(kPatches[0]);
-constexpr int kTkvMax = 14;
+// The patches a thread may own, with the block size their registers allow.
+constexpr ResPatch kPatches[] = {{1, 1, 640}, {2, 1, 512}, {2, 2, 512}, {3, 2, 448}, {4, 2, 384}};
+
+int64_t step_smem(const ResPlan &p, const ResPatch &pt) {
+    const int64_t cells = res_cells(p.gi, p.gj, pt.ri, pt.rj);
+    return 4 * (res_pair_floats((int)cells) + 6LL * p.threads +
+                (2 * cells * res_pitch(kResTkvMax) + 4) * (res_small(pt.ri, pt.rj) ? 2 : 1)) +
+           16LL * (2 * (p.ti + p.tj) * p.tkv + 2 * p.ti * p.tj);
+}
 
 template <int RI, int RJ, int MAXT, bool MIRROR>
 int launch_walled(const ResArgs &a, const ResPlan &p, cudaStream_t st) {
-    static std::mutex mu;
-    static int configured[64] = {0};  // largest dynamic shared memory set so far, per device
-    {
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e != cudaSuccess) return set_cuda_error("cudaGetDevice", e);
-        std::lock_guard<std::mutex> lock(mu);
-        if (dev < 0 || dev >= 64 || p.smem > configured[dev]) {
-            e = cudaFuncSetAttribute(resident_kernel<RI, RJ, kTkvMax, MAXT, MIRROR>, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem);
-            if (e != cudaSuccess) return set_cuda_error("cudaFuncSetAttribute(resident_kernel)", e);
-            if (dev >= 0 && dev < 64) configured[dev] = p.smem;
-        }
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)p.blocks);
-    cfg.blockDim = dim3((unsigned)(p.threads + p.aux));
-    cfg.dynamicSmemBytes = (size_t)p.smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;  // the blocks wait on one another
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, resident_kernel<RI, RJ, kTkvMax, MAXT, MIRROR>, a);
-    if (e != cudaSuccess) return set_cuda_error("cudaLaunchKernelEx(resident_kernel)", e);
-    count_launches(1);
-    return PIC_OK;
+    return launch_cooperative(resident_kernel<RI, RJ, kResTkvMax, MAXT, MIRROR>, "resident_kernel", a, p, st);
 }
-
 template <int RI, int RJ, int MAXT>
 int launch_patch(const ResArgs &a, const ResPlan &p, cudaStream_t st) {
     return a.reflecting ? launch_walled<RI, RJ, MAXT, true>(a, p, st) : launch_walled<RI, RJ, MAXT, false>(a, p, st);
@@ -705,9 +503,9 @@ int next_split(int M, int piece) {
 // 11^2 x 56 to 76^2 x 206 and 59^2 x 406, eleven divisions): a fixed part, the
 // patches (a warp's item takes 65 cycles of its SM, with the larger patches'
 // spills 75), and a round of packets with the faces' size.
-double plan_cost(const ResPlan &p, const Patch &pt) {
+double plan_cost(const ResPlan &p, const ResPatch &pt, double item_scale) {
     const double items = p.threads / 32 * pt.ri * pt.rj;  // of warps
-    double t = 0.4 + (pt.ri * pt.rj >= 6 ? 0.038 : 0.0325) * items;
+    double t = 0.4 + (pt.ri * pt.rj >= 6 ? 0.038 : 0.0325) * item_scale * items;
     if (p.blocks > 1) {
         const double kb = (2.0 * (p.ti + p.tj) * p.tkv * 48.0 + 2.0 * (p.ntk > 1) * p.ti * p.tj * 16.0) / 1024.0;
         t += 0.95 + 0.032 * kb;
@@ -717,14 +515,14 @@ double plan_cost(const ResPlan &p, const Patch &pt) {
     return t;
 }
 
-bool find_plan(int M, int c4, int sms, ResPlan *out) {
+bool find_plan(int M, int c4, int sms, const ResPatch *patches, int count, ResSmem smem_of, double item_scale, ResPlan *out) {
     // more cells than the largest patches hold
     if ((int64_t)M * M * c4 > (int64_t)sms * 4608) return false;
     ResPlan best{};
     double best_t = 1e30;
-    for (int pi = 0; pi < kPatchCount; ++pi) {
-        const Patch &pt = kPatches[pi];
-        for (int ntk = (c4 + kTkvMax - 1) / kTkvMax, tries = 0; tries < 3 && (tries == 0 || c4 / ntk >= 4); ++tries, ++ntk) {
+    for (int pi = 0; pi < count; ++pi) {
+        const ResPatch &pt = patches[pi];
+        for (int ntk = (c4 + kResTkvMax - 1) / kResTkvMax, tries = 0; tries < 3 && (tries == 0 || c4 / ntk >= 4); ++tries, ++ntk) {
             ResPlan p{};
             p.patch = pi;
             p.tkv = (c4 + ntk - 1) / ntk;
@@ -750,12 +548,10 @@ bool find_plan(int M, int c4, int sms, ResPlan *out) {
                     if (left < 1) continue;
                     // a warp beside the chain per 128 patch threads
                     p.aux = 32 * std::min(left, (p.threads + 127) / 128);
-                    const int cells = res_cells(p.gi, p.gj, pt.ri, pt.rj);
-                    const int64_t smem = 4LL * (res_pair_floats(cells) + 6LL * p.threads + (2LL * cells * res_pitch(kTkvMax) + 4) * (res_small(pt.ri, pt.rj) ? 2 : 1)) +
-                                         16LL * (2 * (p.ti + p.tj) * p.tkv + 2 * p.ti * p.tj);
+                    const int64_t smem = smem_of(p, pt);
                     if (smem > kResSmem) continue;
                     p.smem = (int)smem;
-                    const double t = plan_cost(p, pt);
+                    const double t = plan_cost(p, pt, item_scale);
                     if (t < best_t) {
                         best_t = t;
                         best = p;
@@ -772,23 +568,21 @@ bool find_plan(int M, int c4, int sms, ResPlan *out) {
 
 }  // namespace
 
-bool resident_plan(const pic_grid *g, ResPlan *out) {
+bool ResPlanMemo::plan(const pic_grid *g, const ResPatch *patches, int count, ResSmem smem_of, double item_scale,
+                       ResPlan *out) {
     if (g->dtype != PIC_F32 || g->no_xy < 3 || g->no_xy > kResMaxNoXy) return false;
-    const int M = (int)g->no_xy - 2, c4 = (int)(g->kpitch / 4), sms = sm_count();
-    // a segment asks for the plan of its grid again and again: the last one
-    // is kept (it depends on these three numbers alone)
-    struct Last {
-        int M, c4, sms;
-        bool fits;
-        ResPlan plan;
-    };
-    static thread_local Last last{0, 0, 0, false, {}};
-    if (last.M != M || last.c4 != c4 || last.sms != sms) {
-        last = Last{M, c4, sms, false, {}};
-        last.fits = find_plan(M, c4, sms, &last.plan);
+    const int M_ = (int)g->no_xy - 2, c4_ = (int)(g->kpitch / 4), sms_ = sm_count();
+    if (M != M_ || c4 != c4_ || sms != sms_) {
+        M = M_, c4 = c4_, sms = sms_;
+        fits = find_plan(M, c4, sms, patches, count, smem_of, item_scale, &last);
     }
-    if (last.fits) *out = last.plan;
-    return last.fits;
+    if (fits) *out = last;
+    return fits;
+}
+
+bool resident_plan(const pic_grid *g, ResPlan *out) {
+    static thread_local ResPlanMemo memo;
+    return memo.plan(g, kPatches, (int)(sizeof(kPatches) / sizeof(kPatches[0])), step_smem, 1.0, out);
 }
 
 int launch_resident(const pic_grid *g, const ResPlan &p, const void *pos_in, const void *neg_in, void *pos_out,
@@ -804,21 +598,10 @@ int launch_resident(const pic_grid *g, const ResPlan &p, const void *pos_in, con
     a.dens = static_cast<const float2 *>(dens);
     a.dens_stride = dens_stride;
     a.keep_stride = keep_stride;
-    a.packets = static_cast<uint4 *>(packets);
     a.partials = static_cast<float2 *>(partials);
-    a.status = status;
-    a.n = (int)g->no_xy;
-    a.kp = (int)g->kpitch;
-    a.c4 = a.kp / 4;
-    a.nzb = (int)g->nzb;
-    a.nze = (int)g->nze;
-    a.gap_end = (int)(g->nze + g->no_z);
-    a.reflecting = g->wall == PIC_WALL_REFLECTING;
     a.dp = (int)dens_pitch(g->no_xy);
     a.steps = steps;
-    a.nti = p.nti, a.ntj = p.ntj, a.ntk = p.ntk;
-    a.ti = p.ti, a.tj = p.tj, a.tkv = p.tkv, a.gi = p.gi, a.gj = p.gj;
-    a.patch_threads = p.threads, a.aux_threads = p.aux;
+    res_shape(g, p, packets, status, &a);
     a.p_lat = twice((float)g->p_lat), a.p_zm = twice((float)g->p_zm), a.p_zp = twice((float)g->p_zp);
     a.p_cen = twice(centre_weight<float>(g->p_lat, g->p_zm, g->p_zp, g->p_cen));
     a.n_lat = twice((float)g->n_lat), a.n_zm = twice((float)g->n_zm), a.n_zp = twice((float)g->n_zp);

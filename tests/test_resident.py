@@ -165,3 +165,68 @@ def test_what_runs_resident():
     engine = importlib.import_module(pkg().__name__ + ".engine")
     assert engine.runs_resident(engine.make_grid(make_config("column_10um_r008")))
     assert not engine.runs_resident(engine.make_grid(make_config("column_10um_r02", track_cutoff_sigmas=None)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("wall", [0, 1])
+@pytest.mark.parametrize("n,no_z", [(3, 1), (4, 30), (5, 20), (8, 50), (12, 200), (13, 43), (24, 200), (25, 149), (31, 100),
+                                    (48, 200), (53, 200), (48, 400)])
+def test_resident_reverse_sweep_matches_the_float64_one(n, no_z, wall):
+    """lambda over the whole grid, ring and corners included, and the five
+    derivative sums, through segments of even, odd and short lengths.
+
+    Tolerance: lambda as the fields above; a derivative sum adds products mu Du
+    (the last one p n of the scored voxels and mu p n) whose factors are each
+    off by that much of their peaks, so it is off by 2e-6 * steps of the sum of
+    their magnitudes at worst."""
+    import torch
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    lib = native.load()
+    steps, every = 17, 6 if n % 2 else 5
+    rng = np.random.default_rng(7 * n + no_z + wall)
+    kp = (no_z + 4 + 7) // 8 * 8
+    n_seg = -(-steps // every)
+    m = rng.integers(0, 2, steps)
+    m[0] = 1
+    off = np.concatenate([[0], np.cumsum(m)]).astype(np.int64)
+    dp = (n + 3) // 4 * 4
+    ckpt = np.zeros((2, n_seg, n, n, kp))
+    ckpt[..., 1 : no_z + 3] = rng.uniform(0.5, 1.5, (2, n_seg, n, n, no_z + 2))
+    keep = rng.uniform(0.0, 0.1, (int(m.sum()), n, dp, 2))
+
+    def sweep(dtype, variant):
+        g = _grid(native, n, no_z, wall, dtype, variant)
+        t = torch.float64 if dtype == native.PIC_F64 else torch.float32
+        dev = lambda a: torch.from_numpy(a).to("cuda", t)  # noqa: E731
+        c, d = dev(ckpt), dev(keep)
+        states = torch.zeros((2, every, n, n, kp), dtype=t, device="cuda")
+        lam = torch.zeros((2, 2, n, n, kp), dtype=t, device="cuda")
+        grad = torch.zeros(5, dtype=torch.float64, device="cuda")
+        need = {}
+        for name in ("pic_segment_workspace_bytes", "pic_adjoint_workspace_bytes"):
+            b = ctypes.c_int64()
+            native.check(getattr(lib, name)(ctypes.byref(g), ctypes.byref(b)), name)
+            need[name] = torch.zeros(b.value, dtype=torch.uint8, device="cuda")
+        ws, aws = need.values()
+        st = torch.cuda.current_stream().cuda_stream
+        before = lib.pic_kernel_launches()
+        native.check(lib.pic_adjoint_backward(
+            ctypes.byref(g), c[0].data_ptr(), c[1].data_ptr(), n * n * kp, steps, every, off.ctypes.data, d.data_ptr(),
+            states[0].data_ptr(), states[1].data_ptr(), lam[0, 0].data_ptr(), lam[0, 1].data_ptr(), lam[1, 0].data_ptr(),
+            lam[1, 1].data_ptr(), grad.data_ptr(), ws.data_ptr(), ws.numel(), aws.data_ptr(), aws.numel(), st),
+            "pic_adjoint_backward")
+        torch.cuda.synchronize()
+        return lam[steps & 1].double().cpu().numpy(), grad.cpu().numpy(), lib.pic_kernel_launches() - before
+
+    lam, grad, launches = sweep(native.PIC_F32, 0)
+    ref, want, _ = sweep(native.PIC_F64, 1)
+    # two a segment (a short last one step by step) and the final sum; lambda of
+    # the largest does not fit the chip: its adjoint steps are launched one by one
+    assert launches <= 2 * n_seg + 1 + 4 * every + (2 * steps if n * n * no_z > 800000 else 0)
+    tol = 1e-6 * steps
+    for a, b in zip(lam, ref):
+        assert np.abs(a - b).max() <= tol * np.abs(b).max()
+    voxels = steps * (n - 2) ** 2 * (no_z + 2)
+    magnitude = np.array([np.abs(ref).mean() * 2.0] * 4 + [1.0 + np.abs(ref).mean() * 2.0]) * voxels
+    assert (np.abs(grad - want) <= 2 * tol * magnitude).all()
