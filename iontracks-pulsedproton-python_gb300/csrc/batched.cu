@@ -98,25 +98,6 @@ __global__ void batched_prep_kernel(const pic_batch_cfg *cfgs, int n_cfgs, GridE
     table[c] = e;
 }
 
-// Reduction type of a grid's tallies: double-float for float32 fields (no
-// float64 arithmetic), float64 for float64 fields; partial slots are 8 bytes
-// either way.
-template <typename T> struct RedT { using type = double; };
-template <> struct RedT<float> { using type = DF; };
-__device__ __forceinline__ double red_value(double v) { return v; }
-__device__ __forceinline__ double red_value(DF v) { return df_value(v); }
-__device__ __forceinline__ void red_store(double *slot, double v) { *slot = v; }
-__device__ __forceinline__ void red_store(double *slot, DF v) {
-    *reinterpret_cast<float2 *>(slot) = make_float2(v.hi, v.lo);
-}
-__device__ __forceinline__ void red_load_add(double &acc, const double *slot) { acc += __ldcg(slot); }
-__device__ __forceinline__ void red_load_add(DF &acc, const double *slot) {
-    const float2 p = __ldcg(reinterpret_cast<const float2 *>(slot));
-    acc = df_add(acc, DF{p.x, p.y});
-}
-__device__ __forceinline__ double red_of(const Tally<double> &t) { return t.value(); }
-__device__ __forceinline__ DF red_of(const Tally<float> &t) { return df_of(t); }
-
 // One entry of the work table (blk): a range of one grid's items, its
 // tallies reduced per block and, by the grid's last block to finish, into the
 // grid's tally row. `red`, `last` and `a` are the caller's shared memory.

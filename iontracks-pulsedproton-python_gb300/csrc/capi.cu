@@ -268,6 +268,7 @@ static int run_loop(const pic_grid *g, void *pos0, void *neg0, void *pos1, void 
         // the binned deposition of up to kBinSteps steps (kBinTracks tracks)
         // at a time into the workspace's pair buffers, then those steps
         const void *dp[kBinSpan];
+        StepRun run(g, ws, n_steps, st);
         const void *last_pairs = nullptr;  // the pairs of the segment's last step (null: no tracks)
         for (int64_t s0 = 0; s0 < n_steps;) {
             int64_t nd = 0;
@@ -276,8 +277,7 @@ static int run_loop(const pic_grid *g, void *pos0, void *neg0, void *pos1, void 
             if (rc) return rc;
             for (int64_t s = s0; s < s1; ++s) {
                 const int bi = (int)((parity + s) & 1);
-                if ((rc = launch_step(g, pos[bi], neg[bi], pos[bi ^ 1], neg[bi ^ 1], dp[s - s0], nullptr, tally + 4 * s,
-                                      ws, st)))
+                if ((rc = run.step(pos[bi], neg[bi], pos[bi ^ 1], neg[bi ^ 1], dp[s - s0], nullptr, tally + 4 * s)))
                     return rc;
             }
             if (s1 == n_steps) last_pairs = dp[s1 - 1 - s0];
@@ -285,6 +285,7 @@ static int run_loop(const pic_grid *g, void *pos0, void *neg0, void *pos1, void 
         }
         return leave_pairs(g, dens, (int)((dens_parity + n_steps - 1) & 1), last_pairs, st);
     }
+    StepRun run(g, ws, n_steps, st);
     for (int64_t s = 0; s < n_steps; ++s) {
         const int bi = (int)((parity + s) & 1), bo = bi ^ 1;
         const int di = (int)((dens_parity + s) & 1);
@@ -295,8 +296,8 @@ static int run_loop(const pic_grid *g, void *pos0, void *neg0, void *pos1, void 
         }
         // The buffer step s+1 accumulates into was last written at step s-1.
         const bool zero_next = (s == 0) || (off[s] - off[s - 1] > 0);
-        int rc = launch_step(g, pos[bi], neg[bi], pos[bo], neg[bo], m > 0 ? dens[di] : nullptr,
-                             zero_next ? dens[di ^ 1] : nullptr, tally + 4 * s, ws, st);
+        int rc = run.step(pos[bi], neg[bi], pos[bo], neg[bo], m > 0 ? dens[di] : nullptr,
+                          zero_next ? dens[di ^ 1] : nullptr, tally + 4 * s);
         if (rc) return rc;
     }
     return PIC_OK;
@@ -629,6 +630,7 @@ int pic_adjoint_forward(const pic_grid *g, void *pos0, void *neg0, void *pos1, v
         // kept slots
         const void *dp[kBinSpan];
         void *targets[kBinSteps];
+        StepRun run(g, workspace, n_steps, st);
         int64_t d = 0;
         for (int64_t s0 = 0; s0 < n_steps;) {
             int64_t nd = 0;
@@ -640,14 +642,14 @@ int pic_adjoint_forward(const pic_grid *g, void *pos0, void *neg0, void *pos1, v
             for (int64_t s = s0; s < s1; ++s) {
                 const int b = (int)(s & 1);
                 if ((rc = checkpoint(s))) return rc;
-                if ((rc = launch_step(g, pos[b], neg[b], pos[b ^ 1], neg[b ^ 1], dp[s - s0], nullptr, tally + 4 * s,
-                                      workspace, st)))
+                if ((rc = run.step(pos[b], neg[b], pos[b ^ 1], neg[b ^ 1], dp[s - s0], nullptr, tally + 4 * s)))
                     return rc;
             }
             s0 = s1;
         }
         return PIC_OK;
     }
+    StepRun run(g, workspace, n_steps, st);
     int64_t d = 0;
     for (int64_t s = 0; s < n_steps; ++s) {
         const int b = (int)(s & 1);
@@ -668,8 +670,7 @@ int pic_adjoint_forward(const pic_grid *g, void *pos0, void *neg0, void *pos1, v
                                      workspace_bytes)))
                 return rc;
         }
-        rc = launch_step(g, pos[b], neg[b], pos[b ^ 1], neg[b ^ 1], dens, nullptr, tally + 4 * s, workspace, st);
-        if (rc) return rc;
+        if ((rc = run.step(pos[b], neg[b], pos[b ^ 1], neg[b ^ 1], dens, nullptr, tally + 4 * s))) return rc;
     }
     return PIC_OK;
 }

@@ -53,20 +53,6 @@ struct MultiArgs {
     int64_t off[kMaxMultiSteps + 1];  // tracks of step s: [off[s], off[s+1]) of xs/ys
 };
 
-__device__ __forceinline__ double red_of(const Tally<double> &t) { return t.value(); }
-__device__ __forceinline__ DF red_of(const Tally<float> &t) { return df_of(t); }
-__device__ __forceinline__ void red_store(double *slot, double v) { *slot = v; }
-__device__ __forceinline__ void red_store(double *slot, DF v) {
-    *reinterpret_cast<float2 *>(slot) = make_float2(v.hi, v.lo);
-}
-__device__ __forceinline__ void red_load_add(double &acc, const double *slot) { acc += __ldcg(slot); }
-__device__ __forceinline__ void red_load_add(DF &acc, const double *slot) {
-    const float2 p = __ldcg(reinterpret_cast<const float2 *>(slot));
-    acc = df_add(acc, DF{p.x, p.y});
-}
-__device__ __forceinline__ double red_value(double v) { return v; }
-__device__ __forceinline__ double red_value(DF v) { return df_value(v); }
-
 // Block 0: step s's tally from the partials of buffer s & 1 (block order).
 template <typename T>
 __device__ void finish_step(const MultiArgs<T> &p, int s, typename MultiRed<T>::type (*red)[4]) {

@@ -138,6 +138,22 @@ __device__ __forceinline__ DF warp_sum(DF a) {
     return a;
 }
 
+// The sums over a warp of four double-floats at once: each exchange halves
+// the values a lane still carries, so four sums cost 6 additions a lane, not
+// 20. Lane l ends with the sum of v[l >> 3].
+__device__ __forceinline__ DF shfl_df(DF a, int o) {
+    return DF{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
+}
+__device__ __forceinline__ DF warp_sum4(const DF (&v)[4], int lane) {
+    const bool h16 = lane & 16, h8 = lane & 8;
+    const DF a0 = df_add(h16 ? v[2] : v[0], shfl_df(h16 ? v[0] : v[2], 16));
+    const DF a1 = df_add(h16 ? v[3] : v[1], shfl_df(h16 ? v[1] : v[3], 16));
+    DF s = df_add(h8 ? a1 : a0, shfl_df(h8 ? a0 : a1, 8));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s = df_add(s, shfl_df(s, o));
+    return s;
+}
+
 // Block-wide sum of four doubles (or double-floats), result valid in thread
 // 0. Fixed tree order.
 template <int BLOCK, typename A>
@@ -160,27 +176,54 @@ __device__ __forceinline__ void block_sum4(A (&v)[4], A (*smem)[4]) {
     __syncthreads();
 }
 
+// A block's share of a step's four tallies, left at slot[0..3] for a launch
+// that sums them (the next step's, or batched_tallies_kernel).
+template <int BLOCK>
+__device__ __forceinline__ void leave_partial(const DF (&v)[4], double *slot) {
+    constexpr int WARPS = BLOCK / 32;
+    static_assert(WARPS <= 8, "one value a lane");
+    __shared__ DF part[4 * WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const DF s = warp_sum4(v, lane);
+    if ((lane & 7) == 0) part[4 * warp + (lane >> 3)] = s;
+    __syncthreads();
+    if (warp != 0) return;
+    DF x = lane < 4 * WARPS ? part[lane] : DF{0.f, 0.f};
+#pragma unroll
+    for (int o = 4; o < 4 * WARPS; o <<= 1) x = df_add(x, shfl_df(x, o));
+    if (lane < 4) reinterpret_cast<float2 *>(slot)[lane] = make_float2(x.hi, x.lo);
+}
+template <int BLOCK>
+__device__ __forceinline__ void leave_partial(double (&v)[4], double *slot) {
+    __shared__ double red[BLOCK / 32][4];
+    block_sum4<BLOCK>(v, red);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) slot[q] = v[q];
+    }
+}
+
 // The double-float form of finish_tally (below) for float32 kernels: the
 // partials are float2 (hi, lo) pairs in the same 8-byte slots.
 template <int BLOCK>
 __device__ void finish_tally_df(DF (&v)[4], double *partials_d, unsigned int *counter, double *tally,
-                                double injected_scale) {
+                                double injected_scale, unsigned block, unsigned blocks) {
     __shared__ DF red[BLOCK / 32][4];
     __shared__ bool last;
     float2 *partials = reinterpret_cast<float2 *>(partials_d);
     block_sum4<BLOCK>(v, red);
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) partials[4 * (int64_t)blockIdx.x + q] = make_float2(v[q].hi, v[q].lo);
+        for (int q = 0; q < 4; ++q) partials[4 * (int64_t)block + q] = make_float2(v[q].hi, v[q].lo);
         __threadfence();
         unsigned int prev = atomicAdd(counter, 1u);
-        last = (prev == gridDim.x - 1);
+        last = (prev == blocks - 1);
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
     DF acc[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += BLOCK) {
+    for (int b = threadIdx.x; b < (int)blocks; b += BLOCK) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const float2 p = __ldcg(partials + 4 * (int64_t)b + q);
@@ -198,28 +241,62 @@ __device__ void finish_tally_df(DF (&v)[4], double *partials_d, unsigned int *co
     }
 }
 
+// The partials' type and access by field type: double-float for float32 fields
+// (no float64 arithmetic), float64 for float64 fields; 8 bytes either way.
+template <typename T> struct RedT { using type = double; };
+template <> struct RedT<float> { using type = DF; };
+__device__ __forceinline__ double red_of(const Tally<double> &t) { return t.value(); }
+__device__ __forceinline__ DF red_of(const Tally<float> &t) { return df_of(t); }
+__device__ __forceinline__ double red_value(double v) { return v; }
+__device__ __forceinline__ double red_value(DF v) { return df_value(v); }
+__device__ __forceinline__ void red_store(double *slot, double v) { *slot = v; }
+__device__ __forceinline__ void red_store(double *slot, DF v) {
+    *reinterpret_cast<float2 *>(slot) = make_float2(v.hi, v.lo);
+}
+__device__ __forceinline__ void red_load_add(double &acc, const double *slot) { acc += __ldcg(slot); }
+__device__ __forceinline__ void red_load_add(DF &acc, const double *slot) {
+    const float2 p = __ldcg(reinterpret_cast<const float2 *>(slot));
+    acc = df_add(acc, DF{p.x, p.y});
+}
+
+// A step's tally row from its blocks' partials ([parts][4]), by one block.
+template <typename T, int BLOCK>
+__device__ __forceinline__ void sum_partials(const double *partials, int parts, double injected_scale, double *tally) {
+    using R = typename RedT<T>::type;
+    __shared__ R red[BLOCK / 32][4];
+    R v[4] = {R{}, R{}, R{}, R{}};
+    for (int b = threadIdx.x; b < parts; b += BLOCK)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) red_load_add(v[q], partials + 4 * (int64_t)b + q);
+    block_sum4<BLOCK>(v, red);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) tally[q] = red_value(v[q]) * (q == 0 ? injected_scale : 1.0);
+    }
+}
+
 // Completes a step's tallies: every block stores its partial, the last block
-// to finish (completion counter) sums all partials in block order and writes
+// of the step's `blocks` to finish (completion counter) sums all partials in block order and writes
 // tally[0..3]. Deterministic for a given grid size; no float atomics.
 // partial order in memory: {injected (dimensionless), recombined, n+, n-}.
 template <int BLOCK>
 __device__ void finish_tally(double (&v)[4], double *partials, unsigned int *counter, double *tally,
-                             double injected_scale) {
+                             double injected_scale, unsigned block, unsigned blocks) {
     __shared__ double red[BLOCK / 32][4];
     __shared__ bool last;
     block_sum4<BLOCK>(v, red);
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) partials[4 * (int64_t)blockIdx.x + q] = v[q];
+        for (int q = 0; q < 4; ++q) partials[4 * (int64_t)block + q] = v[q];
         __threadfence();
         unsigned int prev = atomicAdd(counter, 1u);
-        last = (prev == gridDim.x - 1);
+        last = (prev == blocks - 1);
     }
     __syncthreads();
     if (!last) return;
     __threadfence();
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += BLOCK) {
+    for (int b = threadIdx.x; b < (int)blocks; b += BLOCK) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[q] += __ldcg(partials + 4 * (int64_t)b + q);
     }

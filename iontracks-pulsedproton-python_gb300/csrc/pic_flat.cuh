@@ -26,6 +26,11 @@ struct StepArgs {
     T p_lat, p_zm, p_zp, p_cen, n_lat, n_zm, n_zp, n_cen, alpha_dt, gfac;
     ScoreTest score;
     double injected_scale;  // no_z: the pairs carry G already
+    // the step before, when its tallies are still to be summed (prev_tally not
+    // null): block 0 sums its prev_blocks partials, the blocks behind it step
+    const double *prev_partials;
+    double *prev_tally;
+    int prev_blocks;
     FastDiv div_c4, div_n;  // item -> column -> (i, j) on the 32-bit path
 };
 

@@ -74,22 +74,6 @@ __device__ __forceinline__ DF two_sum(float a, float b) {
     return DF{s, (a - (s - v)) + (b - v)};
 }
 
-// The sums over a warp of four double-floats at once: each exchange halves
-// the values a lane still carries, so four sums cost 6 additions a lane, not
-// 20. Lane l ends with the sum of v[l >> 3].
-__device__ __forceinline__ DF shfl_df(DF a, int o) {
-    return DF{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
-}
-__device__ __forceinline__ DF warp_sum4(const DF (&v)[4], int lane) {
-    const bool h16 = lane & 16, h8 = lane & 8;
-    const DF a0 = df_add(h16 ? v[2] : v[0], shfl_df(h16 ? v[0] : v[2], 16));
-    const DF a1 = df_add(h16 ? v[3] : v[1], shfl_df(h16 ? v[1] : v[3], 16));
-    DF s = df_add(h8 ? a1 : a0, shfl_df(h8 ? a0 : a1, 8));
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) s = df_add(s, shfl_df(s, o));
-    return s;
-}
-
 // Shared memory: two buffers of deposition pairs over the block's columns (ring
 // and halo included), two buffers of the threads' tallies, one or two buffers
 // of the cells ([row][column][species][4 + 4 TKV] and 4 floats more, a row and a

@@ -299,6 +299,7 @@ int revolve_forward(const pic_grid *g, void *pos0, void *neg0, void *pos1, void 
     const std::vector<Level> sp = spine(n_steps, n_slots);
     void *pos[2] = {pos0, pos1}, *neg[2] = {neg0, neg1};
     size_t q = 0;
+    StepRun run(g, ws, n_steps, st);
     for (int64_t s = 0; s < n_steps; ++s) {
         const int b = (int)(s & 1);
         if (q < sp.size() && sp[q].s0 == s) {
@@ -318,8 +319,7 @@ int revolve_forward(const pic_grid *g, void *pos0, void *neg0, void *pos1, void 
             if (rc) return rc;
             d = dens;
         }
-        int rc = launch_step(g, pos[b], neg[b], pos[b ^ 1], neg[b ^ 1], d, nullptr, tally + 4 * s, ws, st);
-        if (rc) return rc;
+        if (int rc = run.step(pos[b], neg[b], pos[b ^ 1], neg[b ^ 1], d, nullptr, tally + 4 * s)) return rc;
     }
     return PIC_OK;
 }

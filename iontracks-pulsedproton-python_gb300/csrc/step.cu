@@ -1,8 +1,8 @@
 // step.cu -- the fused time step (deposition broadcast + Lax-Wendroff sweep +
 // recombination sink + lateral wall + scored tallies) for one grid.
 //
-// One work item is four consecutive k of one (i, j) column: a 128-bit load or
-// store per species for FP32 fields. Every column of the output is written:
+// One work item is consecutive k of one (i, j) column: eight for FP32 fields
+// (pic_wide.cuh; four beyond 32-bit offsets), four for FP64. Every column of the output is written:
 //   interior (1 <= i, j <= no_xy-2): the 7-point Lax-Wendroff update,
 //     z-weights swapped for the negative species, minus alpha*dt*n+*n-;
 //   outer ring, absorbing wall: the ring is carried with this step's
@@ -25,31 +25,97 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "pic_device.cuh"
 #include "pic_flat.cuh"
 #include "pic_internal.h"
+#include "pic_wide.cuh"
 
 namespace pic {
 
+// The end of a step: the tallies finished here, or (no counter) the block's
+// partials left for the next step's block 0.
+template <int BLOCK>
+__device__ __forceinline__ void end_step(DF (&v)[4], const StepArgs<float> &a, unsigned block, unsigned blocks) {
+    if (a.counter) finish_tally_df<BLOCK>(v, a.partials, a.counter, a.tally, a.injected_scale, block, blocks);
+    else leave_partial<BLOCK>(v, a.partials + 4 * (int64_t)block);
+}
+template <int BLOCK>
+__device__ __forceinline__ void end_step(double (&v)[4], const StepArgs<double> &a, unsigned block, unsigned blocks) {
+    if (a.counter) finish_tally<BLOCK>(v, a.partials, a.counter, a.tally, a.injected_scale, block, blocks);
+    else leave_partial<BLOCK>(v, a.partials + 4 * (int64_t)block);
+}
+
+// The blocks that step: all, or all but block 0, which sums the tallies of the
+// step before (true: done, nothing to step).
+template <typename T, int BLOCK>
+__device__ __forceinline__ bool sums_prev(const StepArgs<T> &a, unsigned &block, unsigned &blocks) {
+    block = blockIdx.x;
+    blocks = gridDim.x;
+    if (!a.prev_tally) return false;
+    if (block == 0) {
+        sum_partials<T, BLOCK>(a.prev_partials, a.prev_blocks, a.injected_scale, a.prev_tally);
+        return true;
+    }
+    --block;
+    --blocks;
+    return false;
+}
+
 template <typename T, int BLOCK, typename I>
 __global__ void __launch_bounds__(BLOCK) step_kernel(StepArgs<T> a) {
+    unsigned block, blocks;
+    if (sums_prev<T, BLOCK>(a, block, blocks)) return;
     Tally<T> t_rec, t_p, t_n, t_inj;
-    const I stride = (I)gridDim.x * BLOCK, items = (I)a.items;
-    for (I item = (I)blockIdx.x * BLOCK + threadIdx.x; item < items; item += stride)
+    const I stride = (I)blocks * BLOCK, items = (I)a.items;
+    for (I item = (I)block * BLOCK + threadIdx.x; item < items; item += stride)
         flat_item<T, I>(a, item, t_rec, t_p, t_n, t_inj);
     if (!a.tally) return;  // no tallies wanted (a recomputation): no reduction
     if constexpr (sizeof(T) == 4) {
         DF v[4] = {df_of(t_inj), df_of(t_rec), df_of(t_p), df_of(t_n)};
-        finish_tally_df<BLOCK>(v, a.partials, a.counter, a.tally, a.injected_scale);
+        end_step<BLOCK>(v, a, block, blocks);
     } else {
         double v[4] = {t_inj.value(), t_rec.value(), t_p.value(), t_n.value()};
-        finish_tally<BLOCK>(v, a.partials, a.counter, a.tally, a.injected_scale);
+        end_step<BLOCK>(v, a, block, blocks);
     }
+}
+
+// The float32 step over eight-wide items (pic_wide.cuh).
+constexpr int kWideBlock = 256, kWideBlocksPerSm = 2;
+__global__ void __launch_bounds__(kWideBlock, kWideBlocksPerSm) wide_step_kernel(StepArgs<float> a) {
+    unsigned block, blocks;
+    if (sums_prev<float, kWideBlock>(a, block, blocks)) return;
+    WideTally tl;
+    wide_sweep(a, a.pos_in, a.neg_in, a.pos_out, a.neg_out, a.dens, a.dens_zero, block * kWideBlock + threadIdx.x,
+               blocks * kWideBlock, tl);
+    if (!a.tally) return;
+    DF v[4];
+    tl.store(v);
+    end_step<kWideBlock>(v, a, block, blocks);
+}
+
+// How a flat step shares its tallies with its neighbours in a run: partials
+// in buffer `slot`, left unsummed (leave), the step before to sum first
+// (prev_tally, prev_blocks; its partials in the other buffer).
+struct StepLink {
+    int slot = 0;
+    bool leave = false;
+    double *prev_tally = nullptr;
+    int prev_blocks = 0;
+};
+
+// Blocks of a flat step (wide: of the eight-wide form); in a run one block
+// fewer than fit at once, so that the summing block runs beside them.
+static int64_t flat_blocks(const pic_grid *g, bool wide, bool run) {
+    const int64_t items = g->no_xy * g->no_xy * (g->kpitch / (wide ? 8 : 4)), block = wide ? kWideBlock : 256;
+    const int64_t cap = wide ? (int64_t)kWideBlocksPerSm * sm_count() : step_grid_cap(g->dtype == PIC_F64 ? 1 : 0);
+    return std::min({(items + block - 1) / block, std::max<int64_t>(1, cap - (run ? 1 : 0)), kMaxStepBlocks / 2});
 }
 
 template <typename T>
 static int launch_step_t(const pic_grid *g, const void *pos_in, const void *neg_in, void *pos_out, void *neg_out,
-                         const void *dens, void *dens_zero, double *tally, void *ws, cudaStream_t st) {
+                         const void *dens, void *dens_zero, double *tally, void *ws, const StepLink *link, cudaStream_t st) {
     constexpr int BLOCK = 256;
     StepArgs<T> a;
     a.pos_in = (const T *)pos_in;
@@ -82,16 +148,38 @@ static int launch_step_t(const pic_grid *g, const void *pos_in, const void *neg_
     a.injected_scale = (double)g->no_z;
     a.div_c4 = make_fastdiv(a.c4);
     a.div_n = make_fastdiv(a.n);
-    int64_t blocks = (a.items + BLOCK - 1) / BLOCK;
-    const int64_t cap = step_grid_cap(g->dtype == PIC_F64 ? 1 : 0);
-    if (blocks > cap) blocks = cap;
-    if (blocks > kMaxStepBlocks) blocks = kMaxStepBlocks;
+    const bool wide = sizeof(T) == 4 && wide_eligible(g->no_xy, g->kpitch, pos_in, neg_in, pos_out, neg_out);
+    int64_t blocks = flat_blocks(g, wide, link);
+    a.prev_partials = nullptr;
+    a.prev_tally = nullptr;
+    a.prev_blocks = 0;
+    if (link) {
+        a.prev_tally = link->prev_tally;
+        a.prev_blocks = link->prev_blocks;
+        a.prev_partials = a.partials + 4 * (link->slot ^ 1) * (kMaxStepBlocks / 2);
+        a.partials += 4 * link->slot * (kMaxStepBlocks / 2);
+        if (link->leave) a.counter = nullptr;
+        if (link->prev_tally) ++blocks;
+    }
+    if constexpr (sizeof(T) == 4) {
+        if (wide) {
+            wide_step_kernel<<<(unsigned)blocks, kWideBlock, 0, st>>>(a);
+            return check_launch("wide_step_kernel");
+        }
+    }
     // (items + stride stays below 2^32 on the 32-bit path: items < 2^29)
     if (flat_index32(g->no_xy, g->kpitch))
         step_kernel<T, BLOCK, uint32_t><<<(unsigned)blocks, BLOCK, 0, st>>>(a);
     else
         step_kernel<T, BLOCK, int64_t><<<(unsigned)blocks, BLOCK, 0, st>>>(a);
     return check_launch("step_kernel");
+}
+
+static int launch_flat(const pic_grid *g, const void *pos_in, const void *neg_in, void *pos_out, void *neg_out,
+                       const void *dens, void *dens_zero, double *tally, void *ws, const StepLink *link, cudaStream_t st) {
+    if (g->dtype == PIC_F64)
+        return launch_step_t<double>(g, pos_in, neg_in, pos_out, neg_out, dens, dens_zero, tally, ws, link, st);
+    return launch_step_t<float>(g, pos_in, neg_in, pos_out, neg_out, dens, dens_zero, tally, ws, link, st);
 }
 
 int launch_step(const pic_grid *g_in, const void *pos_in, const void *neg_in, void *pos_out, void *neg_out,
@@ -104,9 +192,23 @@ int launch_step(const pic_grid *g_in, const void *pos_in, const void *neg_in, vo
         StreamShape sh{g->tile_rows, g->planes_per_item, g->stages, g->consumer_warps, g->ctas_per_sm, sm_count()};
         return launch_stream_step(g, sh, pos_in, neg_in, pos_out, neg_out, dens, dens_zero, tally, ws, st);
     }
-    if (g->dtype == PIC_F64)
-        return launch_step_t<double>(g, pos_in, neg_in, pos_out, neg_out, dens, dens_zero, tally, ws, st);
-    return launch_step_t<float>(g, pos_in, neg_in, pos_out, neg_out, dens, dens_zero, tally, ws, st);
+    return launch_flat(g, pos_in, neg_in, pos_out, neg_out, dens, dens_zero, tally, ws, nullptr, st);
+}
+
+int StepRun::step(const void *pos_in, const void *neg_in, void *pos_out, void *neg_out, const void *dens,
+                  void *dens_zero, double *tally) {
+    if (rc_) return rc_;
+    if (g_.variant == PIC_VARIANT_STREAM)
+        return launch_step(&g_, pos_in, neg_in, pos_out, neg_out, dens, dens_zero, tally, ws_, st_);
+    const bool wide = g_.dtype != PIC_F64 && wide_eligible(g_.no_xy, g_.kpitch, pos_in, neg_in, pos_out, neg_out);
+    StepLink link;
+    link.slot = (int)(left_ & 1);
+    link.leave = --left_ > 0;
+    link.prev_tally = prev_tally_;
+    link.prev_blocks = prev_blocks_;
+    prev_tally_ = link.leave ? tally : nullptr;
+    prev_blocks_ = (int)flat_blocks(&g_, wide, true);
+    return launch_flat(&g_, pos_in, neg_in, pos_out, neg_out, dens, dens_zero, tally, ws_, &link, st_);
 }
 
 int step_occupancy(int dtype, int *blocks_per_sm) {
