@@ -37,17 +37,14 @@ from .feeder import TrackFeeder
 from .pulses import TrackSampler, build_track_schedule
 from .state import Diagnostics, collection_efficiency
 
-# The batched step runs 4 resident 256-thread blocks per SM (float32, 64
-# registers).
-# Items per block are chosen per phase for about WAVES blocks per resident
-# slot on phases of at least SMALL_PHASE_ITEMS items, one block per slot
-# below: few, long blocks amortise each block's set-up and reduction. Measured
-# over the 64-configuration sweep (device ms of the phases with 60-64 / 40-59
-# / 20-39 / 12-19 / 3-11 active grids), blocks per slot 1: 229 / 264 / 251 /
-# 27.0 / 110; 2: 206 / 234 / 210 / 26.5 / 116; 4: 199 / 216 / 204 / 27.5 /
-# 127; 8: 197 / 218 / 211 / 28.8 / 146; 16: 205 / 230 / 228 / 32 / 185.
+# The batched step runs 4 resident blocks per SM (float32: 128 threads, 128
+# registers). Blocks are chosen per phase: WAVES per resident slot on phases of
+# at least SMALL_PHASE_ITEMS items, one per slot below: few, long blocks amortise
+# each block's set-up and reduction. Measured on a 32-configuration sweep (device
+# ms of the first 436 steps, 32 grids of 48.7 M cells), blocks per slot 1: 84.7,
+# 2: 83.2, 4: 86.0, 8: 90.7.
 BLOCKS_PER_SM = 4
-WAVES = 4
+WAVES = 2
 WAVES_SMALL = 1
 SMALL_PHASE_ITEMS = 10_000_000  # four-vector items a step (4e7 voxels)
 MIN_ITEMS_PER_BLOCK = 256
@@ -352,6 +349,21 @@ def _ramp_chunks(phases, chunk_steps: int, first: int = FIRST_CHUNK_STEPS, step_
     return out
 
 
+def _grid_blocks(items, sms: int):
+    """Blocks of each grid of a phase: as many in all as ``items_per_block``
+    means, no more (a block beyond a whole number of waves runs alone at the
+    end of every step: 23 grids of 38.8 M cells took 194 us a step in 616 blocks
+    for 608 slots, 144 us in 607), each further block where the work per block
+    is the largest."""
+    items = np.asarray(items, dtype=np.int64)
+    total = int(items.sum())
+    want = -(-total // items_per_block(total, sms))
+    nb = np.maximum(1, items * want // max(1, total))
+    for _ in range(want - int(nb.sum())):
+        nb[np.argmax(items / nb)] += 1
+    return nb
+
+
 def _work_table(items, active, sms: int) -> dict:
     """Blocks of one batched launch over the ``active`` grids (``items[c]`` =
     grid c's work items): each grid gets contiguous blocks, and block b of a
@@ -359,8 +371,7 @@ def _work_table(items, active, sms: int) -> dict:
     items = np.asarray(items, dtype=np.int64)
     act = np.asarray(active, dtype=np.int64)
     n_cfg = len(items)
-    ipb = items_per_block(int(items[act].sum()), sms)
-    nb = np.maximum(1, -(-items[act] // ipb))
+    nb = _grid_blocks(items[act], sms)
     first = np.concatenate([[0], np.cumsum(nb)[:-1]])
     cfg_blk0 = np.zeros(n_cfg, dtype=np.int32)
     cfg_nblk = np.zeros(n_cfg, dtype=np.int32)

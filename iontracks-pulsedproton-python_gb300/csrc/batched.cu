@@ -9,10 +9,9 @@
 //     over the tracks of every grid: a task list gives each grid's tracks of
 //     the step, each task takes its grid's tiles times its parts of blocks;
 //   * batched_step_kernel -- the flat fused step (pic_flat.cuh) over a work
-//     table that gives each block one grid and a contiguous range of that
-//     grid's items; a grid's blocks are consecutive in the table, and the
-//     last of them to finish (per-grid completion counter) writes the grid's
-//     tallies for this step.
+//     table that gives each block one grid; a grid's blocks are consecutive in
+//     the table and share its items; their partial tallies are summed by one
+//     launch per group of steps.
 // Grids differ in size, time step, coefficients, step count and schedule; a
 // grid that has finished is simply absent from the work table and the task
 // list of later steps (the caller builds one table per set of active grids).
@@ -26,6 +25,7 @@
 #include "pic_barrier.cuh"
 #include "pic_flat.cuh"
 #include "pic_internal.h"
+#include "pic_wide.cuh"
 
 namespace pic {
 
@@ -36,6 +36,7 @@ template <typename T>
 struct GridEntry {
     StepArgs<T> a;
     int64_t field_off, dens_off;
+    int32_t aligned;  // the grid's rows start 32-byte aligned in the packed fields
 };
 
 template <typename T>
@@ -53,6 +54,7 @@ struct BatchStepArgs {
     double *partials; // [n_blocks][4]
     unsigned int *counters;  // [n_cfgs]
     int64_t step;     // global step index (row within each grid's tallies)
+    int aligned;      // the packed fields start 32-byte aligned
 };
 
 template <typename T>
@@ -95,13 +97,15 @@ __global__ void batched_prep_kernel(const pic_batch_cfg *cfgs, int n_cfgs, GridE
     grid_args(cfgs[c], e.a);
     e.field_off = cfgs[c].field_off;
     e.dens_off = cfgs[c].dens_off;
+    e.aligned = e.field_off % 8 == 0 && e.a.kp % 8 == 0;
     table[c] = e;
 }
 
+
 // One entry of the work table (blk): a range of one grid's items, its
-// tallies reduced per block and, by the grid's last block to finish, into the
-// grid's tally row. `red`, `last` and `a` are the caller's shared memory.
-template <typename T, int BLOCK, typename I, bool COH = false>
+// tallies reduced per block and (persistent form), by the grid's last block to
+// finish, into the grid's tally row; else left for batched_tallies_kernel. `red`, `last` and `a` are the caller's shared memory.
+template <typename T, int BLOCK, typename I, bool COH = false, bool WIDE = false>
 __device__ __forceinline__ void batched_step_block(const BatchStepArgs<T> &b, int blk,
                                                    typename RedT<T>::type (*red)[4], bool &last, StepArgs<T> &a) {
     using R = typename RedT<T>::type;
@@ -123,18 +127,37 @@ __device__ __forceinline__ void batched_step_block(const BatchStepArgs<T> &b, in
         }
     }
     __syncthreads();
-    Tally<T> t_rec, t_p, t_n, t_inj;
+    R v[4];
+    bool stepped = false;
+    if constexpr (WIDE) {
+        const GridEntry<T> *E = b.table + c;
+        if (b.aligned && E->aligned) {
+            const int64_t fo = E->field_off, d0 = E->dens_off;
+            WideTally tl;
+            wide_sweep(a, b.pos_in + fo, b.neg_in + fo, b.pos_out + fo, b.neg_out + fo, b.dens + d0,
+                       b.dens_zero ? b.dens_zero + d0 : nullptr, (uint32_t)(blk - b.cfg_blk0[c]) * BLOCK + threadIdx.x,
+                       (uint32_t)b.cfg_nblk[c] * BLOCK, tl);
+            tl.store(v);
+            stepped = true;
+        }
+    }
     // The grid's blocks stride through its items together (block r of nb
     // takes items r*BLOCK + t + k*nb*BLOCK): resident blocks of a grid then
     // sweep one contiguous front through it, and each item's i-1 / i+1
     // neighbours are read while still in L2 (a contiguous chunk per block left
     // hundreds of separate windows in flight across the batch).
-    {
+    if (!stepped) {
+        Tally<T> t_rec, t_p, t_n, t_inj;
         const I r = (I)(blk - b.cfg_blk0[c]), stride = (I)b.cfg_nblk[c] * BLOCK, items = (I)a.items;
         for (I item = r * BLOCK + threadIdx.x; item < items; item += stride)
             flat_item<T, I, COH>(a, item, t_rec, t_p, t_n, t_inj);
+        v[0] = red_of(t_inj), v[1] = red_of(t_rec), v[2] = red_of(t_p), v[3] = red_of(t_n);
     }
-    R v[4] = {red_of(t_inj), red_of(t_rec), red_of(t_p), red_of(t_n)};
+    if constexpr (!COH) {
+        // the launches' tallies: batched_tallies_kernel, a group of steps at once
+        leave_partial<BLOCK>(v, b.partials + 4 * (int64_t)blk);
+        return;
+    }
     block_sum4<BLOCK>(v, red);
     if (threadIdx.x == 0) {
 #pragma unroll
@@ -162,9 +185,14 @@ __device__ __forceinline__ void batched_step_block(const BatchStepArgs<T> &b, in
     }
 }
 
-// float32: four resident blocks per SM (64 registers, a little spilled to
-// local memory) hide more of the heavy phase's global-load latency than three
-// at 80 registers (the 64-grid sweep: 1.12 against 1.15-1.19 s)
+// float32: the eight-wide body (pic_wide.cuh) in four resident blocks of 128
+// threads per SM (128 registers); the work tables count blocks, so smaller ones
+// keep the grids' shares even (blocks of 256, two per SM: 8 to 15 % slower).
+// What bounds it: memory (32 grids of 48.7 M cells stream 780 MB a step from HBM),
+// and the waves' ends. Measured on GB300, us a step, 32 grids of 48.7 M cells / 12
+// of 21.9 M / 3 of 4.3 M: four-wide with each step's last block summing its tallies
+// 212 / 97 / 35; eight-wide 199 / 89 / 29; tallies summed a group of steps at once
+// and two waves of blocks 187 / 86 / 26.
 template <typename T, int BLOCK, typename I>
 __global__ void __launch_bounds__(BLOCK, sizeof(T) == 4 ? 4 : 1) batched_step_kernel(BatchStepArgs<T> b) {
     __shared__ typename RedT<T>::type red[BLOCK / 32][4];
@@ -172,7 +200,20 @@ __global__ void __launch_bounds__(BLOCK, sizeof(T) == 4 ? 4 : 1) batched_step_ke
     // the block's grid arguments, staged once in shared memory and read by
     // broadcast (keeps them out of the registers of every thread)
     __shared__ StepArgs<T> a;
-    batched_step_block<T, BLOCK, I>(b, blockIdx.x, red, last, a);
+    batched_step_block<T, BLOCK, I, false, sizeof(T) == 4 && sizeof(I) == 4>(b, blockIdx.x, red, last, a);
+}
+
+// The tally rows of blockIdx.y consecutive steps of every grid of the work table
+// from its blocks' partials: launched once per group of steps, so that no step
+// ends in a chain of its blocks (store, fence, count, the last block's sum).
+template <typename T>
+__global__ void __launch_bounds__(128) batched_tallies_kernel(const pic_batch_cfg *cfgs, const int32_t *cfg_blk0,
+                                                              const int32_t *cfg_nblk, const double *partials,
+                                                              int64_t n_blocks, int64_t step, double *tally) {
+    const int c = blockIdx.x, nb = cfg_nblk[c];
+    if (nb == 0) return;
+    const double *p = partials + 4 * (n_blocks * blockIdx.y + cfg_blk0[c]);
+    sum_partials<T, 128>(p, nb, (double)cfgs[c].grid.no_z, tally + 4 * (cfgs[c].tally_off + step + blockIdx.y));
 }
 
 // Block `blk` of a global step's deposition (the tile form of
@@ -233,9 +274,10 @@ __device__ __forceinline__ int64_t batched_deposit_blocks(const pic_batch_cfg *c
 // Workspace layout: [per-grid completion counters, n_cfgs x u32, padded to
 // 256 bytes | the persistent kernel's barrier and status, 256 bytes | the
 // prepared grid arguments, n_cfgs slots, padded to 256 bytes | per-block
-// partials, n_blocks x 4 doubles]. The counters sit at a fixed place
+// partials, kTallySteps x n_blocks x 4 doubles]. The counters sit at a fixed place
 // whatever the block count of a launch (which changes when grids finish), so
 // they stay zero between steps.
+constexpr int kTallySteps = 8;  // global steps whose tallies one launch sums
 static int64_t counters_bytes(int32_t n_cfgs) { return ((int64_t)n_cfgs * 4 + 255) / 256 * 256; }
 constexpr int64_t kBarrierBytes = 256;
 
@@ -265,7 +307,7 @@ static double *partials_of(const BatchLaunch &L) {
 
 int batched_workspace_bytes(int32_t n_blocks, int32_t n_cfgs, int64_t *bytes) {
     if (n_blocks < 1 || n_cfgs < 1) return set_error(PIC_E_INVALID, "n_blocks and n_cfgs must be >= 1");
-    *bytes = counters_bytes(n_cfgs) + kBarrierBytes + table_bytes(n_cfgs) + (int64_t)n_blocks * 4 * 8;
+    *bytes = counters_bytes(n_cfgs) + kBarrierBytes + table_bytes(n_cfgs) + (int64_t)kTallySteps * n_blocks * 4 * 8;
     return PIC_OK;
 }
 
@@ -397,10 +439,11 @@ int batched_status(const BatchLaunch &L, cudaStream_t st, int32_t *status) {
 template <typename T, typename I>
 static void launch_batched_step(const BatchLaunch &L, int bi, int bo, double *partials, unsigned int *counters,
                                 int64_t step, cudaStream_t st, const void *dens, void *dens_zero) {
-    constexpr int BLOCK = 256;
+    constexpr int BLOCK = sizeof(T) == 4 && sizeof(I) == 4 ? 128 : 256;
     BatchStepArgs<T> b{L.cfgs, table_of<T>(L), L.blk_cfg, L.blk_item0, L.blk_item1, L.cfg_blk0, L.cfg_nblk,
                        (const T *)L.pos[bi], (const T *)L.neg[bi], (T *)L.pos[bo], (T *)L.neg[bo],
-                       (const pair_t<T> *)dens, (pair_t<T> *)dens_zero, L.tally, partials, counters, step};
+                       (const pair_t<T> *)dens, (pair_t<T> *)dens_zero, L.tally, partials, counters, step,
+                       (((uintptr_t)L.pos[0] | (uintptr_t)L.pos[1] | (uintptr_t)L.neg[0] | (uintptr_t)L.neg[1]) & 31) == 0};
     batched_step_kernel<T, BLOCK, I><<<(unsigned)L.n_blocks, BLOCK, 0, st>>>(b);
 }
 
@@ -559,13 +602,31 @@ int batched_loop(const BatchLaunch &L, cudaStream_t st) { return batched_loop_st
 
 int batched_loop_stream(const BatchLaunch &L, const pic_batch_stream *B, cudaStream_t st) {
     unsigned int *counters = B ? nullptr : reinterpret_cast<unsigned int *>(L.workspace);
-    double *partials = B ? nullptr : partials_of(L);
     if (L.n_steps > 0 && !B) {
         int rc = L.dtype == PIC_F64 ? prep_table<double>(L, st) : prep_table<float>(L, st);
         if (rc) return rc;
     }
+    int waiting = 0;  // steps whose partials wait for their sum
+    int64_t next = 0;
+    auto sum_tallies = [&]() {
+        if (!waiting) return (int)PIC_OK;
+        const dim3 grid((unsigned)L.n_cfgs, (unsigned)waiting);
+        if (L.dtype == PIC_F64)
+            batched_tallies_kernel<double><<<grid, 128, 0, st>>>(L.cfgs, L.cfg_blk0, L.cfg_nblk, partials_of(L),
+                                                                 L.n_blocks, next - waiting, L.tally);
+        else
+            batched_tallies_kernel<float><<<grid, 128, 0, st>>>(L.cfgs, L.cfg_blk0, L.cfg_nblk, partials_of(L),
+                                                                L.n_blocks, next - waiting, L.tally);
+        waiting = 0;
+        return check_launch("batched_tallies_kernel");
+    };
     auto step_launch = [&](int64_t step, int bi, int bo, const void *dens, void *dens_zero) {
         if (B) return batched_stream_step(L, *B, bi, bo, step, dens, dens_zero, st);
+        if (waiting == kTallySteps) {
+            if (int rc = sum_tallies()) return rc;
+        }
+        double *partials = partials_of(L) + 4 * (int64_t)L.n_blocks * waiting++;
+        next = step + 1;
         if (L.dtype == PIC_F64) {
             if (L.index32) launch_batched_step<double, uint32_t>(L, bi, bo, partials, counters, step, st, dens, dens_zero);
             else launch_batched_step<double, int64_t>(L, bi, bo, partials, counters, step, st, dens, dens_zero);
@@ -597,7 +658,7 @@ int batched_loop_stream(const BatchLaunch &L, const pic_batch_stream *B, cudaStr
             }
             s0 = s1;
         }
-        return PIC_OK;
+        return sum_tallies();
     }
     for (int64_t s = 0; s < L.n_steps; ++s) {
         const int64_t step = L.first_step + s;
@@ -620,7 +681,7 @@ int batched_loop_stream(const BatchLaunch &L, const pic_batch_stream *B, cudaStr
         int rc = step_launch(step, bi, bo, L.dens[bi], L.dens[bo]);
         if (rc) return rc;
     }
-    return PIC_OK;
+    return sum_tallies();
 }
 
 }  // namespace pic

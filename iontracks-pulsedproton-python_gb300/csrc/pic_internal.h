@@ -146,8 +146,8 @@ int launch_step(const pic_grid *g, const void *pos_in, const void *neg_in, void 
 // turn) and the next step's block 0 sums them while the others step; the last
 // one finishes its own, so a segment takes no launch more. Measured, us a step
 // of a segment, finished in the step / by the next: 30^2 x 406 9.6 / 6.2, 61^2 x 606
-// 14.4 / 10.3, 119^2 x 406 22.7 / 18.8, 208^2 x 406 57.0 / 53.3; float64 36^2 x 206
-// 28 / 24. The streaming step finishes its own.
+// 14.4 / 10.3, 119^2 x 406 22.7 / 19.6, 208^2 x 406 57.0 / 53.3; float64 36^2 x 206
+// 26.7 / 22.6. The streaming step finishes its own.
 class StepRun {
 public:
     StepRun(const pic_grid *g, void *ws, int64_t steps, cudaStream_t st) : g_(*g), ws_(ws), st_(st), left_(steps) {

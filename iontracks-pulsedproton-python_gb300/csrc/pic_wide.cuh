@@ -15,8 +15,8 @@
 // columns a thread (fewer loads a cell), prefetches of the next pass into L2 and
 // planes marched in registers measured no faster. Measured on GB300, us a step of
 // a segment without tracks, four-wide / here (the tallies' share in pic_internal.h):
-// 30^2 x 406 9.6 / 6.2, 61^2 x 606 14.4 / 10.3, 119^2 x 406 26.0 / 18.8, 208^2 x 406
-// 60.5 / 53.3, 330^2 x 406 137.5 / 123.5, 608^2 x 406 449 / 412; with 1500 tracks a
+// 30^2 x 406 9.6 / 6.2, 61^2 x 606 14.4 / 10.3, 119^2 x 406 26.0 / 19.6, 208^2 x 406
+// 60.5 / 53.3, 330^2 x 406 137.5 / 124.2, 608^2 x 406 449 / 412; with 1500 tracks a
 // step, their deposition included, 208^2 x 406 68.9 / 59.0.
 #pragma once
 
@@ -63,22 +63,21 @@ __device__ __forceinline__ uint32_t spread(uint32_t m) {
 __device__ __forceinline__ float keep(float v, uint32_t m) { return __uint_as_float(__float_as_uint(v) & m); }
 __device__ __forceinline__ float2 keep2(float2 v, const uint32_t *m) { return {keep(v.x, m[0]), keep(v.y, m[1])}; }
 
-// Two Kahan running sums side by side (Tally<float>), one packed operation
-// for both.
+// Two running sums side by side as double-floats s + c, each addition Knuth's
+// TwoSum in packed operations (a - b as fma(b, -1, a), the same rounding): the
+// sums do not depend on how the items fall to threads beyond 2^-44.
 struct Tally2 {
     float2 s = {0.f, 0.f}, c = {0.f, 0.f};
     __device__ __forceinline__ void add(float2 v) {
-        const float2 y = __fadd2_rn(v, float2{-c.x, -c.y});
-        const float2 t = __fadd2_rn(s, y);
-        const float2 u = __fadd2_rn(t, float2{-s.x, -s.y});
-        c = __fadd2_rn(u, float2{-y.x, -y.y});
+        const float2 m1 = {-1.f, -1.f};
+        const float2 t = __fadd2_rn(s, v), z = __ffma2_rn(s, m1, t);
+        const float2 e = __ffma2_rn(__ffma2_rn(z, m1, t), m1, s);
+        c = __fadd2_rn(c, __fadd2_rn(e, __ffma2_rn(z, m1, v)));
         s = t;
     }
 };
 __device__ __forceinline__ DF df_of(const Tally2 &t) {
-    Tally<float> a, b;
-    a.s = t.s.x, a.c = t.c.x, b.s = t.s.y, b.c = t.c.y;
-    return df_add(df_of(a), df_of(b));
+    return df_add(DF{t.s.x, t.c.x}, DF{t.s.y, t.c.y});
 }
 
 struct WideTally {

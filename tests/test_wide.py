@@ -4,11 +4,12 @@ tallies a segment's steps sum for one another, against the float64 step.
 Tolerance as for the resident step: 1e-6 of the peak a step, steps added up."""
 
 import importlib
+import warnings
 
 import numpy as np
 import pytest
 
-from goldens import make_config, pkg
+from goldens import pkg
 from test_resident import _case, _compare, _grid, _segment
 
 # no_xy, no_z (four layers more in all): one interior column; a column of one
@@ -34,3 +35,39 @@ def test_flat_segment_matches_the_float64_step(n, no_z, wall):
             got = _segment(native, g, torch, state, xs, ys, off, n & 1)
             ref = _segment(native, g64, torch, state, xs, ys, off, n & 1)
             _compare(native, got, ref, steps)
+
+
+def _thick_batch():
+    kw = dict(grid_size_um=10.0, E_MeV_u=56.2, dose_rate_Gy_s=20.0, pulse_duration_s=4e-7, repetition_rate_hz=50.0)
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        return [pkg().SimulationConfig(voltage_V=v, electrode_gap_cm=gap, sampled_radius_cm=r, seed=s, **kw)
+                for v, gap, r, s in ((4000.0, 1.2, 0.002, 1), (3000.0, 0.2, 0.006, 2), (3500.0, 0.1, 0.012, 3))]
+
+
+@pytest.mark.gpu
+def test_batched_steps_do_not_depend_on_the_blocks(monkeypatch):
+    """Grids with fewer threads than vectors in a column (one block for 1206
+    layers), and with one block or many: the same fields, bit for bit, and the
+    same tallies to the rounding of their double-float sums (44 bits)."""
+    batched = importlib.import_module(pkg().__name__ + ".batched")
+    run = lambda: pkg().run_batched_b200(_thick_batch(), solo_grids=0, return_fields=True)
+    many = run()
+    monkeypatch.setattr(batched, "_grid_blocks", lambda items, sms: np.ones(len(items), dtype=np.int64))
+    for a, b in zip(many, run()):
+        assert np.array_equal(a.positive_array, b.positive_array) and np.array_equal(a.negative_array, b.negative_array)
+        assert np.abs(a.positive_array).max() > 0
+        np.testing.assert_allclose(a.recombination, b.recombination, rtol=1e-11, atol=0)
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_grid_blocks_fill_whole_waves(seed):
+    batched = importlib.import_module(pkg().__name__ + ".batched")
+    rng = np.random.default_rng(seed)
+    items = rng.integers(300, 3_000_000, int(rng.integers(1, 64)))
+    nb = batched._grid_blocks(items, 152)
+    want = -(-int(items.sum()) // batched.items_per_block(int(items.sum()), 152))
+    assert nb.min() >= 1 and nb.sum() <= max(want, want + (nb == 1).sum() - 1)
+    if (items * want // items.sum()).min() >= 1:
+        assert nb.sum() == want
+        assert (items / nb).max() <= 2 * items.sum() / want
