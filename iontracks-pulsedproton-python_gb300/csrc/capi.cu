@@ -218,10 +218,6 @@ static int leave_pairs(const pic_grid *g, void *const dens[2], int last, const v
     return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaMemsetAsync(deposition pairs)", e);
 }
 
-static cudaError_t clear_bin_counts(const pic_grid *g, void *ws, cudaStream_t st) {
-    return cudaMemsetAsync(static_cast<char *>(ws) + kWorkspaceBytes, 0, (size_t)bin_count_bytes(g->no_xy), st);
-}
-
 static int run_loop(const pic_grid *g, void *pos0, void *neg0, void *pos1, void *neg1, int64_t parity,
                     int64_t n_steps, const double *xs, const double *ys, const int64_t *off, void *dens0,
                     void *dens1, int64_t dens_parity, uint32_t *counts, double *tally, void *ws,
@@ -262,25 +258,22 @@ static int run_loop(const pic_grid *g, void *pos0, void *neg0, void *pos1, void 
     int64_t most = 0;
     for (int64_t s = 0; s < n_steps; ++s) most = std::max(most, off[s + 1] - off[s]);
     if (most > 0 && most <= kBinTracks && deposit_binned(g, ws, ws_bytes, most)) {
-        // (another grid may have left its own lists where this one's counts are)
-        cudaError_t e = clear_bin_counts(g, ws, st);
-        if (e != cudaSuccess) return set_cuda_error("cudaMemsetAsync(tile counts)", e);
-        // the binned deposition of up to kBinSteps steps (kBinTracks tracks)
-        // at a time into the workspace's pair buffers, then those steps
-        const void *dp[kBinSpan];
+        // the binned deposition of a group of steps at a time into the
+        // workspace's pair buffers, then those steps
+        StepDeposits dep(g, xs, ys, off, counts, ws, ws_bytes, st);
         StepRun run(g, ws, n_steps, st);
         const void *last_pairs = nullptr;  // the pairs of the segment's last step (null: no tracks)
+        int rc = dep.begin();
+        if (rc) return rc;
         for (int64_t s0 = 0; s0 < n_steps;) {
-            int64_t nd = 0;
-            const int64_t s1 = next_deposit_group(off, s0, n_steps, &nd);
-            int rc = launch_deposit_steps(g, xs, ys, off, s0, s1, counts, ws, nullptr, dp, st);
-            if (rc) return rc;
+            int64_t s1 = s0, nd = 0;
+            if ((rc = dep.group(s0, n_steps, nullptr, 0, &s1, &nd))) return rc;
             for (int64_t s = s0; s < s1; ++s) {
                 const int bi = (int)((parity + s) & 1);
-                if ((rc = run.step(pos[bi], neg[bi], pos[bi ^ 1], neg[bi ^ 1], dp[s - s0], nullptr, tally + 4 * s)))
+                if ((rc = run.step(pos[bi], neg[bi], pos[bi ^ 1], neg[bi ^ 1], dep.pairs[s - s0], nullptr, tally + 4 * s)))
                     return rc;
             }
-            if (s1 == n_steps) last_pairs = dp[s1 - 1 - s0];
+            if (s1 == n_steps) last_pairs = dep.pairs[s1 - 1 - s0];
             s0 = s1;
         }
         return leave_pairs(g, dens, (int)((dens_parity + n_steps - 1) & 1), last_pairs, st);
@@ -416,7 +409,8 @@ int pic_segment_workspace_bytes(const pic_grid *g, int64_t *bytes) {
     if (rc) return rc;
     if (!bytes) return set_error(PIC_E_INVALID, "bytes is null");
     ResPlan plan;
-    *bytes = resident_plan(g, &plan) ? resident_space(g, plan).end : kWorkspaceBytes + dep_bin_bytes(g);
+    *bytes = std::max(kWorkspaceBytes + dep_bin_bytes(g), ahead_space(g).end);
+    if (resident_plan(g, &plan)) *bytes = std::max(*bytes, resident_space(g, plan).end);
     return PIC_OK;
 }
 
@@ -624,25 +618,19 @@ int pic_adjoint_forward(const pic_grid *g, void *pos0, void *neg0, void *pos1, v
     int64_t most = 0;
     for (int64_t s = 0; s < n_steps; ++s) most = std::max(most, track_offsets[s + 1] - track_offsets[s]);
     if (most > 0 && most <= kBinTracks && deposit_binned(g, workspace, workspace_bytes, most)) {
-        cudaError_t e = clear_bin_counts(g, workspace, st);
-        if (e != cudaSuccess) return set_cuda_error("cudaMemsetAsync(tile counts)", e);
-        // each launch pair deposits up to kBinSteps steps straight into their
-        // kept slots
-        const void *dp[kBinSpan];
-        void *targets[kBinSteps];
+        // each launch pair deposits a group of steps straight into their kept slots
+        StepDeposits dep(g, xs, ys, track_offsets, counts, workspace, workspace_bytes, st);
         StepRun run(g, workspace, n_steps, st);
+        if ((rc = dep.begin())) return rc;
         int64_t d = 0;
         for (int64_t s0 = 0; s0 < n_steps;) {
-            int64_t nd = 0;
-            const int64_t s1 = next_deposit_group(track_offsets, s0, n_steps, &nd);
-            for (int64_t k = 0; k < nd; ++k) targets[k] = D + (d + k) * dslot * es;
-            if ((rc = launch_deposit_steps(g, xs, ys, track_offsets, s0, s1, counts, workspace, targets, dp, st)))
-                return rc;
+            int64_t s1 = s0, nd = 0;
+            if ((rc = dep.group(s0, n_steps, D + d * dslot * es, dslot * es, &s1, &nd))) return rc;
             d += nd;
             for (int64_t s = s0; s < s1; ++s) {
                 const int b = (int)(s & 1);
                 if ((rc = checkpoint(s))) return rc;
-                if ((rc = run.step(pos[b], neg[b], pos[b ^ 1], neg[b ^ 1], dp[s - s0], nullptr, tally + 4 * s)))
+                if ((rc = run.step(pos[b], neg[b], pos[b ^ 1], neg[b ^ 1], dep.pairs[s - s0], nullptr, tally + 4 * s)))
                     return rc;
             }
             s0 = s1;

@@ -30,6 +30,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "pic_binned.cuh"
 #include "pic_deposit.cuh"
 #include "pic_device.cuh"
@@ -204,10 +206,11 @@ int launch_deposit_steps(const pic_grid *g, const double *xs, const double *ys, 
                                : launch_binned_steps<float>(g, xs, ys, off, s0, s1, counts, ws, targets, dens, st);
 }
 
-int launch_deposit_slots(const pic_grid *g, const double *xs, const double *ys, const int64_t *off, int64_t s0,
-                         int64_t s1, uint32_t *hist, void *ws, const ResSpace &r, void *dens, int64_t dens_stride,
-                         int16_t *slot, cudaStream_t st) {
-    BinSlotsSteps<float> S{};
+template <typename T>
+static int launch_slots(const pic_grid *g, const double *xs, const double *ys, const int64_t *off, int64_t s0,
+                        int64_t s1, uint32_t *hist, void *ws, int64_t counts, int64_t lists, void *dens,
+                        int64_t dens_stride, int16_t *slot, cudaStream_t st) {
+    BinSlotsSteps<T> S{};
     int k = 0;
     for (int64_t s = s0; s < s1; ++s) {
         slot[s - s0] = -1;
@@ -221,20 +224,68 @@ int launch_deposit_slots(const pic_grid *g, const double *xs, const double *ys, 
     S.tracks = off[s1] - off[s0];
     S.off[k] = (int32_t)S.tracks;
     if (S.tracks > kBinTracks) return set_error(PIC_E_INVALID, "more than kBinTracks tracks in one launch");
-    DepBins<float> bins = dep_bins<float>(ws, g->no_xy);
+    DepBins<T> bins = dep_bins<T>(ws, g->no_xy);
     char *w = static_cast<char *>(ws);
-    bins.count = reinterpret_cast<int *>(w + r.counts);
-    bins.list = reinterpret_cast<int *>(w + r.lists);
-    S.base = grid_slot<float>(g, bins, 0, xs + off[s0], ys + off[s0], 0, S.tracks, dens, hist, 0);
+    bins.count = reinterpret_cast<int *>(w + counts);
+    bins.list = reinterpret_cast<int *>(w + lists);
+    S.base = grid_slot<T>(g, bins, 0, xs + off[s0], ys + off[s0], 0, S.tracks, dens, hist, 0);
     S.dens_stride = dens_stride;
-    return binned_launches<float>(S, bins.scratch, k * bins.tiles, st);
+    return binned_launches<T>(S, bins.scratch, k * bins.tiles, st);
 }
 
-int64_t next_deposit_group(const int64_t *off, int64_t s0, int64_t n_steps, int64_t *n_dep) {
+int launch_deposit_slots(const pic_grid *g, const double *xs, const double *ys, const int64_t *off, int64_t s0,
+                         int64_t s1, uint32_t *hist, void *ws, int64_t counts, int64_t lists, void *dens,
+                         int64_t dens_stride, int16_t *slot, cudaStream_t st) {
+    return g->dtype == PIC_F64
+               ? launch_slots<double>(g, xs, ys, off, s0, s1, hist, ws, counts, lists, dens, dens_stride, slot, st)
+               : launch_slots<float>(g, xs, ys, off, s0, s1, hist, ws, counts, lists, dens, dens_stride, slot, st);
+}
+
+AheadSpace ahead_space(const pic_grid *g) {
+    const int64_t es = g->dtype == PIC_F64 ? 8 : 4, tiles = bin_tiles_per_side(g->no_xy) * bin_tiles_per_side(g->no_xy);
+    AheadSpace a{};
+    if (!bin_eligible(g) || g->deposit_variant != PIC_DEPOSIT_AUTO) return a;
+    const int64_t want = (kAheadBlocksPerSm * sm_count() + tiles - 1) / tiles;
+    if (want <= kBinSteps) return a;
+    a.slots = (int)std::min<int64_t>(want, kResSteps);
+    a.counts = kWorkspaceBytes + dep_bin_bytes(g);
+    a.lists = a.counts + bin_align(a.slots * tiles * 4);
+    a.dens = a.lists + a.slots * tiles * kBinCap * 4;
+    a.end = a.dens + a.slots * bin_dens_bytes(g->no_xy, es);
+    return a;
+}
+
+int StepDeposits::begin() {
+    const int64_t tiles = bin_tiles_per_side(g_->no_xy) * bin_tiles_per_side(g_->no_xy);
+    // (another grid may have left its own lists where this one's counts are)
+    const cudaError_t e = space_.slots
+        ? cudaMemsetAsync(static_cast<char *>(ws_) + space_.counts, 0, (size_t)(space_.slots * tiles * 4), st_)
+        : cudaMemsetAsync(static_cast<char *>(ws_) + kWorkspaceBytes, 0, (size_t)bin_count_bytes(g_->no_xy), st_);
+    return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaMemsetAsync(tile counts)", e);
+}
+
+int StepDeposits::group(int64_t s0, int64_t n_steps, char *targets, int64_t target_bytes, int64_t *s1, int64_t *n_dep) {
+    *s1 = next_deposit_group(off_, s0, n_steps, space_.slots ? space_.slots : kBinSteps, n_dep);
+    const int64_t es = g_->dtype == PIC_F64 ? 8 : 4;
+    if (space_.slots) {
+        int16_t slot[kBinSpan];
+        char *dens = targets ? targets : static_cast<char *>(ws_) + space_.dens;
+        const int64_t stride = targets ? target_bytes : bin_dens_bytes(g_->no_xy, es);
+        int rc = launch_deposit_slots(g_, xs_, ys_, off_, s0, *s1, counts_, ws_, space_.counts, space_.lists, dens,
+                                      stride / (2 * es), slot, st_);
+        for (int64_t s = s0; s < *s1; ++s) pairs[s - s0] = slot[s - s0] < 0 ? nullptr : dens + slot[s - s0] * stride;
+        return rc;
+    }
+    void *at[kBinSteps];
+    for (int64_t k = 0; k < *n_dep && targets; ++k) at[k] = targets + k * target_bytes;
+    return launch_deposit_steps(g_, xs_, ys_, off_, s0, *s1, counts_, ws_, targets ? at : nullptr, pairs, st_);
+}
+
+int64_t next_deposit_group(const int64_t *off, int64_t s0, int64_t n_steps, int slots, int64_t *n_dep) {
     int64_t s1 = s0, nd = 0;
     while (s1 < n_steps && s1 - s0 < kBinSpan) {
         const int64_t m = off[s1 + 1] - off[s1];
-        if (m > 0 && (nd == kBinSteps || off[s1 + 1] - off[s0] > kBinTracks)) break;
+        if (m > 0 && (nd == slots || off[s1 + 1] - off[s0] > kBinTracks)) break;
         nd += m > 0;
         ++s1;
     }

@@ -306,19 +306,20 @@ int resident_steps(const pic_grid *g, const ResPlan &plan, const void *pos_in, c
                    void *neg_out, const double *xs, const double *ys, const int64_t *off, int64_t s0, int64_t s1,
                    uint32_t *counts, double *tally, void *targets, int64_t target_stride, const void **last_pairs,
                    void *ws, cudaStream_t st);
-// The binned deposition of the steps of one resident launch, a slot per step
-// with tracks; slot[s - s0] receives step s's (-1: none).
+// The binned deposition of steps s0 .. s1 - 1 (up to kResSteps with tracks),
+// a slot per step with tracks; slot[s - s0] receives step s's (-1: none). counts
+// and lists: the slots' tile counts (zero) and lists, byte offsets in ws.
 int launch_deposit_slots(const pic_grid *g, const double *xs, const double *ys, const int64_t *off, int64_t s0,
-                         int64_t s1, uint32_t *hist, void *ws, const ResSpace &r, void *dens, int64_t dens_stride,
-                         int16_t *slot, cudaStream_t st);
+                         int64_t s1, uint32_t *hist, void *ws, int64_t counts, int64_t lists, void *dens,
+                         int64_t dens_stride, int16_t *slot, cudaStream_t st);
 
 // Whether the deposition takes the binned form for this grid and workspace:
 // for a segment's steps together (most = the most tracks one of them has),
 // or with most < 0 for one step alone.
 bool deposit_binned(const pic_grid *g, const void *ws, int64_t ws_bytes, int64_t most);
-// The end of the next launch pair's steps from s0: at most kBinSteps of them
+// The end of the next launch pair's steps from s0: at most `slots` of them
 // with tracks (*n_dep), kBinTracks tracks and kBinSpan steps.
-int64_t next_deposit_group(const int64_t *off, int64_t s0, int64_t n_steps, int64_t *n_dep);
+int64_t next_deposit_group(const int64_t *off, int64_t s0, int64_t n_steps, int slots, int64_t *n_dep);
 // The binned deposition of steps s0 .. s1 - 1 (tracks xs/ys[off[s] ..
 // off[s + 1]), a group of next_deposit_group) into targets[k] for the k-th
 // step with tracks, or with targets null into the workspace's pair buffers:
@@ -400,5 +401,47 @@ int arrival_counts_pcg64(uint64_t *st, int64_t n, double duration, const double 
                          int64_t *counts);
 int sample_disc_pcg64(uint64_t *st, double scale, double mid, double radius_sq, int64_t n_wanted, int64_t max_pairs,
                       double *xs, double *ys, int64_t *n_accepted, int64_t *n_draws);
+
+// Deposition further ahead than kBinSteps steps, for grids of few tiles whose
+// eight steps leave most SMs without a block (a 36^2 grid: 8 blocks, one of them
+// 59 us in float64): as many steps a launch pair as give kAheadBlocksPerSm blocks
+// an SM, at most kResSteps, in slots of their own behind the step workspace. Only
+// where the choice of deposition is the library's and the workspace is
+// pic_segment_workspace_bytes large. slots = 0: not for this grid. Measured, us a
+// step, eight steps a pair / ahead: float32 119^2 x 406 with 70 tracks 22.4 / 20.8,
+// 208^2 x 406 with 300 57.5 / 55.9, with 1500 60.5 / 57.3, 330^2 x 206 with 500
+// 70.4 / 69.4; a whole float64 run of 36^2 x 206 (2097 steps, 39 tracks each) 65.1
+// / 50.7 ms.
+constexpr int kAheadBlocksPerSm = 4;
+struct AheadSpace {
+    int64_t counts, lists, dens, end;  // byte offsets from the workspace's start
+    int slots;
+};
+AheadSpace ahead_space(const pic_grid *g);
+
+// The binned depositions of a segment, group by group.
+class StepDeposits {
+public:
+    StepDeposits(const pic_grid *g, const double *xs, const double *ys, const int64_t *off, uint32_t *counts, void *ws,
+                 int64_t ws_bytes, cudaStream_t st)
+        : g_(g), xs_(xs), ys_(ys), off_(off), counts_(counts), ws_(ws), st_(st), space_(ahead_space(g)) {
+        if (ws_bytes < space_.end) space_.slots = 0;
+    }
+    int begin();  // before the segment's first group
+    // Deposits the next group's steps [s0, *s1), *n_dep of them with tracks:
+    // the k-th of these into targets + k * target_bytes (targets null: into the
+    // workspace); pairs[s - s0]: step s's pairs, null without tracks.
+    int group(int64_t s0, int64_t n_steps, char *targets, int64_t target_bytes, int64_t *s1, int64_t *n_dep);
+    const void *pairs[kBinSpan];
+
+private:
+    const pic_grid *g_;
+    const double *xs_, *ys_;
+    const int64_t *off_;
+    uint32_t *counts_;
+    void *ws_;
+    cudaStream_t st_;
+    AheadSpace space_;
+};
 
 }  // namespace pic

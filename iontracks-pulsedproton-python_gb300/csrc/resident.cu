@@ -637,7 +637,7 @@ int resident_steps(const pic_grid *g, const ResPlan &plan, const void *pos_in, c
     char *dens = targets ? static_cast<char *>(targets) : w + r.dens;
     const int64_t stride = targets ? target_stride : bin_dens_bytes(g->no_xy, 4) / 8;
     int16_t slot[kResSteps];
-    int rc = launch_deposit_slots(g, xs, ys, off, s0, s1, counts, ws, r, dens, stride, slot, st);
+    int rc = launch_deposit_slots(g, xs, ys, off, s0, s1, counts, ws, r.counts, r.lists, dens, stride, slot, st);
     if (rc) return rc;
     const int16_t end = slot[s1 - 1 - s0];
     *last_pairs = end < 0 ? nullptr : dens + 8 * stride * end;

@@ -71,3 +71,22 @@ def test_grid_blocks_fill_whole_waves(seed):
     if (items * want // items.sum()).min() >= 1:
         assert nb.sum() == want
         assert (items / nb).max() <= 2 * items.sum() / want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["PIC_F32", "PIC_F64"])
+@pytest.mark.parametrize("n,no_z,steps", [(20, 3, 300), (200, 3, 90)])
+def test_depositing_further_ahead_changes_nothing(n, no_z, steps, dtype):
+    """Segments with more depositing steps than the slots of one launch pair (256
+    for one tile, 38 for sixteen), against groups of eight: the same bits."""
+    import torch
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    state, xs, ys, off = _case(n, no_z, steps, n, 40)
+    g = _grid(native, n, no_z, 0, getattr(native, dtype), native.PIC_VARIANT_FLAT)
+    runs = [_segment(native, g, torch, state, xs, ys, off, 0, workspace=w)
+            for w in ("pic_segment_workspace_bytes", "pic_step_workspace_bytes")]
+    for a, b in zip(runs[0][:5], runs[1][:5]):
+        assert np.array_equal(a, b)
+    for a, b in zip(runs[0][5], runs[1][5]):
+        assert np.array_equal(a, b)
