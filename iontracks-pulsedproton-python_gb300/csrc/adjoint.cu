@@ -370,7 +370,7 @@ int adjoint_workspace_bytes(int64_t *bytes) {
 static int64_t adjoint_blocks(const pic_grid *g) {
     const int64_t items = g->no_xy * g->no_xy * (g->kpitch / 4);
     int64_t blocks = (items + 255) / 256;
-    const int64_t cap = step_grid_cap(g->dtype == PIC_F64 ? 1 : 0);
+    const int64_t cap = g->dtype == PIC_F64 ? 2 * (int64_t)sm_count() : step_grid_cap(0);
     if (blocks > cap) blocks = cap;
     if (blocks > kMaxStepBlocks) blocks = kMaxStepBlocks;
     return blocks;

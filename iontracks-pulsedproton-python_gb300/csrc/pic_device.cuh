@@ -193,14 +193,28 @@ __device__ __forceinline__ void leave_partial(const DF (&v)[4], double *slot) {
     for (int o = 4; o < 4 * WARPS; o <<= 1) x = df_add(x, shfl_df(x, o));
     if (lane < 4) reinterpret_cast<float2 *>(slot)[lane] = make_float2(x.hi, x.lo);
 }
-template <int BLOCK>
-__device__ __forceinline__ void leave_partial(double (&v)[4], double *slot) {
-    __shared__ double red[BLOCK / 32][4];
-    block_sum4<BLOCK>(v, red);
-    if (threadIdx.x == 0) {
+// (float64 additions are what a warp waits for: 6 a lane here, not 20)
+__device__ __forceinline__ double warp_sum4(const double (&v)[4], int lane) {
+    const bool h16 = lane & 16, h8 = lane & 8;
+    const double a0 = (h16 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16);
+    const double a1 = (h16 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h16 ? v[1] : v[3], 16);
+    double s = (h8 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h8 ? a0 : a1, 8);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) slot[q] = v[q];
-    }
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+template <int BLOCK>
+__device__ __forceinline__ void leave_partial(const double (&v)[4], double *slot) {
+    __shared__ double part[BLOCK / 32][4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double s = warp_sum4(v, lane);
+    if ((lane & 7) == 0) part[warp][lane >> 3] = s;
+    __syncthreads();
+    if (threadIdx.x >= 4) return;
+    double x = part[0][threadIdx.x];
+#pragma unroll
+    for (int w = 1; w < BLOCK / 32; ++w) x += part[w][threadIdx.x];
+    slot[threadIdx.x] = x;
 }
 
 // The double-float form of finish_tally (below) for float32 kernels: the

@@ -113,6 +113,11 @@ __device__ __forceinline__ void flat_item(const StepArgs<T> &a, I item, Tally<T>
         return;
     }
 
+    const I dcol = ci * dp + cj;
+    // this column's deposition and its neighbours' (gap layers only): one
+    // pair per column, in flight with the fields
+    pair_t<T> d{T(0), T(0)};
+    if (a.dens) d = ld1<COH>(a.dens + dcol);
     const I ccol = ci * n + cj;
     const I base = ccol * kp + k0;
     const I di = n * kp;
@@ -126,23 +131,24 @@ __device__ __forceinline__ void flat_item(const StepArgs<T> &a, I item, Tally<T>
     T pkp = k0 + 4 < kp ? ld1<COH>(a.pos_in + base + 4) : T(0);
     T nkp = k0 + 4 < kp ? ld1<COH>(a.neg_in + base + 4) : T(0);
 
-    const I dcol = ci * dp + cj;
-    // this column's deposition and its neighbours' (gap layers only): one
-    // pair per column
-    T dc = T(0), dl = T(0);
+    V4<T> LP, LN;  // the lateral neighbours' sums
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        LP.v[e] = (Pjm.v[e] + Pjp.v[e]) + (Pim.v[e] + Pip.v[e]);
+        LN.v[e] = (Njm.v[e] + Njp.v[e]) + (Nim.v[e] + Nip.v[e]);
+    }
     if (a.dens) {
-        const pair_t<T> d = ld1<COH>(a.dens + dcol);
-        dc = d.x;
-        dl = d.y;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             if (g[e]) {
-                P.v[e] += dc;
-                N.v[e] += dc;
+                P.v[e] += d.x;
+                N.v[e] += d.x;
+                LP.v[e] += d.y;
+                LN.v[e] += d.y;
             }
         }
-        if (g_km) { pkm += dc; nkm += dc; }
-        if (g_kp) { pkp += dc; nkp += dc; }
+        if (g_km) { pkm += d.x; nkm += d.x; }
+        if (g_kp) { pkp += d.x; nkp += d.x; }
     }
 
     const bool scored_col = !ring && scored_col_t<I>(a.score, ci, cj);
@@ -156,19 +162,16 @@ __device__ __forceinline__ void flat_item(const StepArgs<T> &a, I item, Tally<T>
         const T p_kp1 = e < 3 ? P.v[e + 1] : pkp;
         const T n_km1 = e > 0 ? N.v[e - 1] : nkm;
         const T n_kp1 = e < 3 ? N.v[e + 1] : nkp;
-        const T dle = g[e] ? dl : T(0);
-        const T p_new = a.p_zm * p_km1 + a.p_zp * p_kp1 +
-                        a.p_lat * (((Pjm.v[e] + Pjp.v[e]) + (Pim.v[e] + Pip.v[e])) + dle) + a.p_cen * p;
-        const T n_new = a.n_zm * n_kp1 + a.n_zp * n_km1 +
-                        a.n_lat * (((Njm.v[e] + Njp.v[e]) + (Nim.v[e] + Nip.v[e])) + dle) + a.n_cen * nn;
-        const T rec = a.alpha_dt * p * nn;
+        const T p_new = a.p_zm * p_km1 + a.p_zp * p_kp1 + a.p_lat * LP.v[e] + a.p_cen * p;
+        const T n_new = a.n_zm * n_kp1 + a.n_zp * n_km1 + a.n_lat * LN.v[e] + a.n_cen * nn;
+        const T ap = a.alpha_dt * p;
         const bool valid = (k >= 1) && (k <= a.nzb - 2);
-        const T po = valid ? p_new - rec : T(0);
-        const T no = valid ? n_new - rec : T(0);
+        const T po = valid ? fma(-ap, nn, p_new) : T(0);
+        const T no = valid ? fma(-ap, nn, n_new) : T(0);
         PO.v[e] = po;
         NO.v[e] = no;
         if (scored_col && g[e]) {
-            rec_sum += rec;
+            rec_sum = fma(ap, nn, rec_sum);
             p_sum += po;
             n_sum += no;
         }
@@ -179,7 +182,7 @@ __device__ __forceinline__ void flat_item(const StepArgs<T> &a, I item, Tally<T>
         t_rec.add(rec_sum);
         t_p.add(p_sum);
         t_n.add(n_sum);
-        if (c == 0 && a.dens) t_inj.add(dc);
+        if (c == 0 && a.dens) t_inj.add(d.x);
     }
 }
 

@@ -105,10 +105,17 @@ struct StepLink {
     int prev_blocks = 0;
 };
 
+// Threads of a four-wide block. Float64 steps of a small grid are bound by the
+// FP64 units, which an SM shares among its warps: small blocks spread the warps
+// evenly (36^2 x 206: 264 blocks of 256 leave 40 of 152 SMs half the work of the
+// rest). Measured with 90 tracks a step, us a step: 64 threads 19.7, 128 and 256
+// 21.7, 32 23.8; 100^2 x 406 164 either way.
+template <typename T> constexpr int kFlatBlock = sizeof(T) == 8 ? 64 : 256;
+
 // Blocks of a flat step (wide: of the eight-wide form); in a run one block
 // fewer than fit at once, so that the summing block runs beside them.
 static int64_t flat_blocks(const pic_grid *g, bool wide, bool run) {
-    const int64_t items = g->no_xy * g->no_xy * (g->kpitch / (wide ? 8 : 4)), block = wide ? kWideBlock : 256;
+    const int64_t items = g->no_xy * g->no_xy * (g->kpitch / (wide ? 8 : 4)), block = wide ? kWideBlock : g->dtype == PIC_F64 ? kFlatBlock<double> : kFlatBlock<float>;
     const int64_t cap = wide ? (int64_t)kWideBlocksPerSm * sm_count() : step_grid_cap(g->dtype == PIC_F64 ? 1 : 0);
     return std::min({(items + block - 1) / block, std::max<int64_t>(1, cap - (run ? 1 : 0)), kMaxStepBlocks / 2});
 }
@@ -116,7 +123,7 @@ static int64_t flat_blocks(const pic_grid *g, bool wide, bool run) {
 template <typename T>
 static int launch_step_t(const pic_grid *g, const void *pos_in, const void *neg_in, void *pos_out, void *neg_out,
                          const void *dens, void *dens_zero, double *tally, void *ws, const StepLink *link, cudaStream_t st) {
-    constexpr int BLOCK = 256;
+    constexpr int BLOCK = kFlatBlock<T>;
     StepArgs<T> a;
     a.pos_in = (const T *)pos_in;
     a.neg_in = (const T *)neg_in;
@@ -213,7 +220,7 @@ int StepRun::step(const void *pos_in, const void *neg_in, void *pos_out, void *n
 
 int step_occupancy(int dtype, int *blocks_per_sm) {
     cudaError_t e = dtype == PIC_F64
-                        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel<double, 256, uint32_t>, 256, 0)
+                        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel<double, kFlatBlock<double>, uint32_t>, kFlatBlock<double>, 0)
                         : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel<float, 256, uint32_t>, 256, 0);
     return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaOccupancyMaxActiveBlocksPerMultiprocessor", e);
 }
