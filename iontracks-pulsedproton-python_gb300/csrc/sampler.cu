@@ -127,7 +127,7 @@ int sample_disc_pcg64(uint64_t *st, double scale, double mid, double radius_sq, 
 // (pcg_advance); the sum then runs once over them in place; and since a_k
 // never decreases in k, bin b's count is the distance between the first
 // index whose a_k reaches edges[b] and the first reaching edges[b + 1]
-// (binary searches). Small pulses take one sequential pass instead.
+// (binary searches). Smaller pulses are drawn by one thread.
 namespace {
 
 constexpr int64_t kArrivalThreadedMin = (int64_t)1 << 20;
@@ -153,6 +153,100 @@ void arrival_counts_serial(Pcg64 start, int64_t n, double duration, const double
     end = r;
 }
 
+// One thread: the draws of kArrivalBlock at a time in four interleaved chains (the
+// state's 128-bit multiply-add is the longest chain, four draws apart its maps are
+// independent), added up in order; the sum and the state before each block are
+// kept, and a block an edge falls into is drawn again. One division per search
+// step instead of one per draw. On the GB300's host, into 2 948 bins, drawn twice /
+// in blocks: 888 000 draws 3.39 / 1.56 ms, 300 000 1.19 / 0.71, 69 000 0.33 / 0.33,
+// 5 000 0.07 / 0.11: worth it from about 32 draws a bin.
+constexpr int kArrivalBlock = 32;
+
+void arrival_counts_blocks(Pcg64 start, int64_t n, double duration, const double *edges, int64_t n_edges,
+                           int64_t *counts, Pcg64 &end) {
+    const int64_t blocks = (n + kArrivalBlock - 1) / kArrivalBlock, nb = n_edges - 1;
+    std::vector<double> before((size_t)blocks + 1);
+    std::vector<u128> state((size_t)blocks);
+    const u128 m2 = kPcgMult * kPcgMult, c2 = (kPcgMult + 1) * start.inc, m4 = m2 * m2, c4 = (m2 + 1) * c2;
+    auto output = [](u128 s) {
+        const uint64_t x = (uint64_t)(s >> 64) ^ (uint64_t)s;
+        const unsigned rot = (unsigned)(s >> 122);
+        return (double)(((x >> rot) | (x << ((64u - rot) & 63u))) >> 11) * (1.0 / 9007199254740992.0);
+    };
+    // adds draws [0, m) of the block that starts in state s to sum; s moves on
+    auto add_block = [&](u128 &s, double sum, int m, double *sums) {
+        u128 q[4];
+        q[0] = s * kPcgMult + start.inc;
+        for (int e = 1; e < 4; ++e) q[e] = q[e - 1] * kPcgMult + start.inc;
+        int k = 0;
+        for (; k + 4 <= m; k += 4) {
+            double u[4];
+            for (int e = 0; e < 4; ++e) u[e] = output(q[e]);
+            s = q[3];
+            for (int e = 0; e < 4; ++e) q[e] = q[e] * m4 + c4;
+            for (int e = 0; e < 4; ++e) {
+                sum += u[e];
+                if (sums) sums[k + e] = sum;
+            }
+        }
+        for (int e = 0; k < m; ++k, ++e) {
+            s = q[e];
+            sum += output(s);
+            if (sums) sums[k] = sum;
+        }
+        return sum;
+    };
+    u128 s = start.state;
+    double sum = 0.0;
+    for (int64_t b = 0; b < blocks; ++b) {
+        before[b] = sum;
+        state[b] = s;
+        sum = add_block(s, sum, (int)std::min<int64_t>(kArrivalBlock, n - b * kArrivalBlock), nullptr);
+    }
+    before[blocks] = sum;
+    const double last = sum;
+    auto reaches = [&](double S, double e, bool strict) {
+        const double q = S / last;
+        const double t = q * duration;
+        return strict ? t > e : t >= e;
+    };
+    double sums[kArrivalBlock];
+    int64_t drawn = -1, at = 0;  // the block in sums; the block of the last edge
+    auto first_at = [&](double e, bool strict) {
+        // the first block whose last arrival reaches e (edges ascend)
+        int64_t lo = at, hi = blocks;
+        for (int64_t w = 1; lo + w < hi; w *= 2) {
+            if (reaches(before[lo + w], e, strict)) { hi = lo + w; break; }
+        }
+        while (lo < hi) {
+            const int64_t mid = lo + (hi - lo) / 2;
+            if (reaches(before[mid + 1], e, strict)) hi = mid; else lo = mid + 1;
+        }
+        if (lo == blocks) return n;
+        at = lo;
+        const int m = (int)std::min<int64_t>(kArrivalBlock, n - lo * kArrivalBlock);
+        if (drawn != lo) {
+            u128 q = state[lo];
+            add_block(q, before[lo], m, sums);
+            drawn = lo;
+        }
+        int k = 0, kh = m - 1;
+        while (k < kh) {
+            const int mid = (k + kh) / 2;
+            if (reaches(sums[mid], e, strict)) kh = mid; else k = mid + 1;
+        }
+        return lo * kArrivalBlock + k;
+    };
+    int64_t prev = first_at(edges[0], false);
+    for (int64_t b = 0; b < nb; ++b) {
+        const int64_t next = b + 1 < nb ? first_at(edges[b + 1], false) : first_at(edges[nb], true);
+        counts[b] = next > prev ? next - prev : 0;
+        prev = next > prev ? next : prev;
+    }
+    end.state = s;
+    end.inc = start.inc;
+}
+
 }  // namespace
 
 int arrival_counts_pcg64(uint64_t *st, int64_t n, double duration, const double *edges, int64_t n_edges,
@@ -163,7 +257,8 @@ int arrival_counts_pcg64(uint64_t *st, int64_t n, double duration, const double 
     const unsigned hw = std::thread::hardware_concurrency();
     const int64_t threads = std::min<int64_t>(std::max<unsigned>(hw, 1u), 64);
     if (n < kArrivalThreadedMin || threads < 2) {
-        arrival_counts_serial(start, n, duration, edges, n_edges, counts, end);
+        if (n >= 32 * n_edges) arrival_counts_blocks(start, n, duration, edges, n_edges, counts, end);
+        else arrival_counts_serial(start, n, duration, edges, n_edges, counts, end);
     } else {
         std::unique_ptr<double[]> S(new double[(size_t)n]);
         double *u = S.get();

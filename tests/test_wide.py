@@ -5,6 +5,7 @@ Tolerance as for the resident step: 1e-6 of the peak a step, steps added up."""
 
 import importlib
 import warnings
+from types import SimpleNamespace
 
 import numpy as np
 import pytest
@@ -90,3 +91,20 @@ def test_depositing_further_ahead_changes_nothing(n, no_z, steps, dtype):
         assert np.array_equal(a, b)
     for a, b in zip(runs[0][5], runs[1][5]):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,bins", [(31, 1), (32, 1), (33, 1), (64, 1), (97, 2), (130, 3), (1025, 31), (70001, 400)])
+def test_arrivals_drawn_in_blocks_equal_numpys(n, bins):
+    """The histogram of a pulse drawn in blocks (from 32 draws a bin on), and the
+    generator's place after it, with bins that end before, at and past the pulse."""
+    pulses = importlib.import_module(pkg().__name__ + ".pulses")
+    for seed, end in ((1, 0.97), (2, 1.0), (3, 1.05)):
+        edges = np.linspace(0.0, 5.4e-4 * end, bins + 1)
+        cfg = SimpleNamespace(number_of_tracks_per_pulse=n, pulse_duration_s=5.4e-4, pulse_time_bins=edges)
+        mine, theirs = np.random.default_rng(seed), np.random.default_rng(seed)
+        got = pulses.pulse_arrival_counts(cfg, mine)
+        arrival = np.cumsum(theirs.random(n))
+        arrival /= arrival[-1]
+        arrival *= cfg.pulse_duration_s
+        assert np.array_equal(got, np.histogram(arrival, edges)[0])
+        assert mine.random() == theirs.random()
