@@ -49,6 +49,7 @@
 #include "pic_device.cuh"
 #include "pic_flat.cuh"
 #include "pic_internal.h"
+#include "pic_wide.cuh"
 
 namespace pic {
 
@@ -88,6 +89,47 @@ __device__ __forceinline__ void block_sum_n(A (&v)[kAdjGrad], A (*smem)[kAdjGrad
 #pragma unroll
         for (int q = 0; q < kAdjGrad; ++q) v[q] = warp_sum(lane < BLOCK / 32 ? smem[lane][q] : A{});
     __syncthreads();
+}
+
+// The end of an adjoint step: the block's sums into its running slots
+// (accumulate), or the step's totals by the last block to finish.
+template <typename T, int BLOCK>
+__device__ __forceinline__ void finish_adjoint(typename AdjRed<T>::type (&v)[kAdjGrad],
+                                               typename AdjRed<T>::type (*red)[kAdjGrad], bool &last,
+                                               const AdjArgs<T> &a) {
+    using R = typename AdjRed<T>::type;
+    block_sum_n<BLOCK>(v, red);
+    if (a.accumulate) {
+        // the backward sweep needs only the sum over steps: each block keeps
+        // its own running sums (same block, same slot, every step; launches
+        // are ordered on the stream), reduced once at the end
+        if (threadIdx.x == 0)
+#pragma unroll
+            for (int q = 0; q < kAdjGrad; ++q) adj_accumulate(a.partials + (int64_t)kAdjGrad * blockIdx.x + q, v[q]);
+        return;
+    }
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < kAdjGrad; ++q) adj_store(a.partials + (int64_t)kAdjGrad * blockIdx.x + q, v[q]);
+        __threadfence();
+        last = (atomicAdd(a.counter, 1u) == gridDim.x - 1);
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    R s[kAdjGrad];
+#pragma unroll
+    for (int q = 0; q < kAdjGrad; ++q) s[q] = R{};
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += BLOCK)
+#pragma unroll
+        for (int q = 0; q < kAdjGrad; ++q) adj_load_add(s[q], a.partials + (int64_t)kAdjGrad * b + q);
+    block_sum_n<BLOCK>(s, red);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < kAdjGrad; ++q) a.grad[q] = adj_value(s[q]);
+        *a.counter = 0u;
+        __threadfence();
+    }
 }
 
 // u~ (with this step's deposition on gap layers) of four k at column offset
@@ -255,38 +297,198 @@ __global__ void __launch_bounds__(BLOCK) adjoint_step_kernel(AdjArgs<T> a) {
     R v[kAdjGrad];
 #pragma unroll
     for (int q = 0; q < kAdjGrad; ++q) v[q] = adj_of(acc[q]);
-    block_sum_n<BLOCK>(v, red);
-    if (a.accumulate) {
-        // the backward sweep needs only the sum over steps: each block keeps
-        // its own running sums (same block, same slot, every step; launches
-        // are ordered on the stream), reduced once at the end
-        if (threadIdx.x == 0)
+    finish_adjoint<T, BLOCK>(v, red, last, a);
+}
+
+__device__ __forceinline__ Oct zero8() { return Oct{{{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}}}; }
+__device__ __forceinline__ float2 twice(float x) { return {x, x}; }
+__device__ __forceinline__ float2 minus2(float2 a, float2 b) { return __ffma2_rn(b, float2{-1.f, -1.f}, a); }
+
+// The adjoint step of a float32 grid over eight-wide items (threads, columns, k
+// neighbours and ring items as in pic_wide.cuh), the derivative sums by parts
+// (adjoint_stream.cu), so that of the state only the voxels themselves are read:
+// 12 eight-wide loads an item where the four-wide kernel takes 26 loads for half
+// as much. 157 registers, 12 warps an SM. What bounds it: memory (208^2 x 406
+// moves 424 MB a step, 61 us at the measured copy rate). Measured on GB300 with
+// tracks, us a step, four-wide / here / streaming: 62^2 x 206 16.6 / 12.5 / 84,
+// 119^2 x 406 65.8 / 37.4 / 67.7, 208^2 x 406 174 / 93.9 / 125, 330^2 x 406
+// 428 / 221 / 236, 608^2 x 406 1503 / 728 / 718.
+constexpr int kWideAdjBlock = 128, kWideAdjBlocksPerSm = 3;
+__global__ void __launch_bounds__(kWideAdjBlock, kWideAdjBlocksPerSm) wide_adjoint_kernel(AdjArgs<float> a) {
+    constexpr int BLOCK = kWideAdjBlock;
+    __shared__ DF red[BLOCK / 32][kAdjGrad];
+    __shared__ bool last;
+    Tally2 acc[kAdjGrad];
+    const uint32_t n = (uint32_t)a.n, kp = (uint32_t)a.kp, c8 = kp / 8, dp = (uint32_t)a.dp, di = n * kp, w = n - 2;
+    const uint32_t inner = w * w, all = n * n, r = blockIdx.x * BLOCK + threadIdx.x, T = gridDim.x * BLOCK;
+    const bool many = T >= c8;
+    const uint32_t step = many ? T / c8 : 1;
+    const uint32_t step_i = step / w, step_j = step - step_i * w;
+    const uint32_t at_step = (step_i * n + step_j) * kp;
+    const int lane = threadIdx.x & 31, two_mid = (int)a.score.two_mid;
+    const bool scores = a.score.thr4 >= 0;
+    const uint32_t thr = a.score.thr4 >= 0xffffffffLL ? 0xffffffffu : (uint32_t)a.score.thr4;
+    const float2 half = twice(0.5f), m1 = twice(-1.f), m2 = twice(-2.f), m6 = twice(-6.f);
+
+    for (uint32_t pass = 0;; ++pass) {
+        const uint32_t col0 = many ? r / c8 : 0;
+        uint32_t c = many ? r - col0 * c8 : pass * T + r;
+        const bool ok = many ? col0 < step : c < c8;
+        if (!__any_sync(0xffffffffu, ok)) break;
+        if (!ok) c = c8 - 1;
+        const int k0 = (int)(8 * c);
+        uint32_t g_lo = 0, g_hi = 0, v_lo = 0, v_hi = 0;
 #pragma unroll
-            for (int q = 0; q < kAdjGrad; ++q) adj_accumulate(a.partials + (int64_t)kAdjGrad * blockIdx.x + q, v[q]);
-        return;
+        for (int e = 0; e < 4; ++e) {
+            const uint32_t bit = 0x80u << (8 * e);
+            const int k = k0 + e, q = k0 + 4 + e;
+            g_lo |= (k >= a.nze && k < a.gap_end) ? bit : 0u;
+            g_hi |= (q >= a.nze && q < a.gap_end) ? bit : 0u;
+            v_lo |= (k >= 1 && k <= a.nzb - 2) ? bit : 0u;
+            v_hi |= (q >= 1 && q <= a.nzb - 2) ? bit : 0u;
+        }
+        const bool ends = (v_lo & v_hi) != 0x80808080u, edge_lane = lane == 0 || lane == 31;
+        const uint32_t edge_off = lane == 0 ? 0xffffffffu : 8u;
+        uint32_t v = ok ? col0 : all;
+        uint32_t i = ok ? 1 + col0 / w : 1, j = ok ? 1 + col0 - (i - 1) * w : 1;
+        uint32_t at = (i * n + j) * kp + (uint32_t)k0;
+        while (__any_sync(0xffffffffu, v < inner)) {
+            const bool act = v < inner;
+            const uint32_t base = act ? at : n * kp + kp + (uint32_t)k0;
+            float2 d = {0.f, 0.f};
+            if (a.dens) d = __ldg(a.dens + (act ? i * dp + j : dp + 1));
+            const Oct MP = load8(a.lp + base), MN = load8(a.ln + base);
+            Oct LP = zero8(), LN = zero8();
+            {
+                // mu is zero on the ring
+                const bool up = act && i > 1, down = act && i < w, left = act && j > 1, right = act && j < w;
+                const Oct A0 = up ? load8(a.lp + (base - di)) : zero8(), B0 = up ? load8(a.ln + (base - di)) : zero8();
+                const Oct A1 = down ? load8(a.lp + (base + di)) : zero8(), B1 = down ? load8(a.ln + (base + di)) : zero8();
+                const Oct A2 = left ? load8(a.lp + (base - kp)) : zero8(), B2 = left ? load8(a.ln + (base - kp)) : zero8();
+                const Oct A3 = right ? load8(a.lp + (base + kp)) : zero8(), B3 = right ? load8(a.ln + (base + kp)) : zero8();
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    LP.v[h] = __fadd2_rn(__fadd2_rn(A0.v[h], A1.v[h]), __fadd2_rn(A2.v[h], A3.v[h]));
+                    LN.v[h] = __fadd2_rn(__fadd2_rn(B0.v[h], B1.v[h]), __fadd2_rn(B2.v[h], B3.v[h]));
+                }
+            }
+            const Oct P = load8(a.pos + base), N = load8(a.neg + base);
+            float ep = 0.f, en = 0.f;
+            if (edge_lane) {
+                ep = __ldg(a.lp + (base + edge_off));
+                en = __ldg(a.ln + (base + edge_off));
+            }
+            // (mu is zero on a column's end layers and padding, so the value
+            // of a lane that holds another column's end is right here)
+            float mp_km = __shfl_up_sync(0xffffffffu, MP.v[3].y, 1), mn_km = __shfl_up_sync(0xffffffffu, MN.v[3].y, 1);
+            float mp_kp = __shfl_down_sync(0xffffffffu, MP.v[0].x, 1), mn_kp = __shfl_down_sync(0xffffffffu, MN.v[0].x, 1);
+            if (lane == 0) mp_km = ep, mn_km = en;
+            if (lane == 31) mp_kp = ep, mn_kp = en;
+            const uint32_t m[8] = {spread<0>(g_lo), spread<1>(g_lo), spread<2>(g_lo), spread<3>(g_lo),
+                                   spread<0>(g_hi), spread<1>(g_hi), spread<2>(g_hi), spread<3>(g_hi)};
+            const int dx = 2 * (int)i - two_mid, dy = 2 * (int)j - two_mid;
+            const bool scored = scores && (uint32_t)(dx * dx) + (uint32_t)(dy * dy) <= thr;
+            float2 G0 = {0.f, 0.f}, G1 = G0, G2 = G0, G3 = G0, G4 = G0;
+            Oct OP, ON;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const float2 mp = MP.v[h], mn = MN.v[h];
+                const float2 mpd = {h > 0 ? MP.v[h > 0 ? h - 1 : 0].y : mp_km, mp.x};
+                const float2 mpu = {mp.y, h < 3 ? MP.v[h < 3 ? h + 1 : 3].x : mp_kp};
+                const float2 mnd = {h > 0 ? MN.v[h > 0 ? h - 1 : 0].y : mn_km, mn.x};
+                const float2 mnu = {mn.y, h < 3 ? MN.v[h < 3 ? h + 1 : 3].x : mn_kp};
+                float2 p = P.v[h], q = N.v[h];
+                if (a.dens) {
+                    const float2 D = keep2(twice(d.x), m + 2 * h), L = keep2(twice(d.y), m + 2 * h);
+                    p = __fadd2_rn(p, D);
+                    q = __fadd2_rn(q, D);
+                    G0 = __ffma2_rn(mp, L, G0);
+                    G2 = __ffma2_rn(mn, L, G2);
+                }
+                const float2 S = __fadd2_rn(mp, mn);
+                const float2 AN = __fmul2_rn(twice(a.a), q), AP = __fmul2_rn(twice(a.a), p), pn = __fmul2_rn(p, q);
+                float2 lp = __ffma2_rn(twice(a.p_cen), mp, __ffma2_rn(twice(a.p_lat), LP.v[h],
+                            __ffma2_rn(twice(a.p_zp), mpd, __fmul2_rn(twice(a.p_zm), mpu))));
+                float2 ln = __ffma2_rn(twice(a.n_cen), mn, __ffma2_rn(twice(a.n_lat), LN.v[h],
+                            __ffma2_rn(twice(a.n_zp), mnu, __fmul2_rn(twice(a.n_zm), mnd))));
+                const float2 nS = __fmul2_rn(S, m1);
+                lp = __ffma2_rn(AN, nS, lp);
+                ln = __ffma2_rn(AP, nS, ln);
+                G4 = __ffma2_rn(nS, pn, G4);
+                if (scored) {
+                    lp = __fadd2_rn(lp, keep2(AN, m + 2 * h));
+                    ln = __fadd2_rn(ln, keep2(AP, m + 2 * h));
+                    G4 = __fadd2_rn(G4, keep2(pn, m + 2 * h));
+                }
+                OP.v[h] = lp;
+                ON.v[h] = ln;
+                const float2 zp = __fadd2_rn(mpu, mpd), zn = __fadd2_rn(mnu, mnd);
+                G0 = __ffma2_rn(P.v[h], LP.v[h], __ffma2_rn(p, __ffma2_rn(m6, mp, zp), G0));
+                G2 = __ffma2_rn(N.v[h], LN.v[h], __ffma2_rn(q, __ffma2_rn(m6, mn, zn), G2));
+                G1 = __ffma2_rn(p, __ffma2_rn(twice(a.c_pos), __ffma2_rn(m2, mp, zp), __fmul2_rn(half, minus2(mpu, mpd))), G1);
+                G3 = __ffma2_rn(q, __ffma2_rn(twice(a.c_neg), __ffma2_rn(m2, mn, zn), __fmul2_rn(half, minus2(mnd, mnu))), G3);
+            }
+            if (ends) {
+                const uint32_t u[8] = {spread<0>(v_lo), spread<1>(v_lo), spread<2>(v_lo), spread<3>(v_lo),
+                                       spread<0>(v_hi), spread<1>(v_hi), spread<2>(v_hi), spread<3>(v_hi)};
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    OP.v[h] = keep2(OP.v[h], u + 2 * h);
+                    ON.v[h] = keep2(ON.v[h], u + 2 * h);
+                }
+            }
+            if (act) {
+                store8(a.lp_out + base, OP);
+                store8(a.ln_out + base, ON);
+                acc[0].add(G0);
+                acc[1].add(G1);
+                acc[2].add(G2);
+                acc[3].add(G3);
+                acc[4].add(G4);
+                v += step;
+                at += at_step;
+                i += step_i;
+                j += step_j;
+                if (j > w) j -= w, ++i, at += 2 * kp;
+            }
+        }
+        // ring: lat mu of the column beside it (none beside a corner), and
+        // its own lambda where the wall absorbs; its state, in that
+        // column's lateral sum
+        for (; v < all; v += step) {
+            const uint32_t u = v - inner;
+            if (u < 2 * n) i = u < n ? 0 : n - 1, j = u < n ? u : u - n;
+            else i = 1 + (u - 2 * n) / 2, j = (u & 1) ? n - 1 : 0;
+            const uint32_t o = (i * n + j) * kp + (uint32_t)k0;
+            const bool corner = (i == 0 || i == n - 1) && (j == 0 || j == n - 1);
+            Oct OP = zero8(), ON = zero8();
+            if (!a.reflecting) {
+                OP = load8(a.lp + o);
+                ON = load8(a.ln + o);
+            }
+            if (!corner) {
+                const uint32_t b = i == 0 ? o + di : i == n - 1 ? o - di : j == 0 ? o + kp : o - kp;
+                const Oct MP = load8(a.lp + b), MN = load8(a.ln + b), P = load8(a.pos + o), N = load8(a.neg + o);
+                float2 G0 = {0.f, 0.f}, G2 = G0;
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    OP.v[h] = __ffma2_rn(twice(a.p_lat), MP.v[h], OP.v[h]);
+                    ON.v[h] = __ffma2_rn(twice(a.n_lat), MN.v[h], ON.v[h]);
+                    G0 = __ffma2_rn(P.v[h], MP.v[h], G0);
+                    G2 = __ffma2_rn(N.v[h], MN.v[h], G2);
+                }
+                acc[0].add(G0);
+                acc[2].add(G2);
+            }
+            store8(a.lp_out + o, OP);
+            store8(a.ln_out + o, ON);
+        }
+        if (many) break;
     }
-    if (threadIdx.x == 0) {
+    DF s[kAdjGrad];
 #pragma unroll
-        for (int q = 0; q < kAdjGrad; ++q) adj_store(a.partials + (int64_t)kAdjGrad * blockIdx.x + q, v[q]);
-        __threadfence();
-        last = (atomicAdd(a.counter, 1u) == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    R s[kAdjGrad];
-#pragma unroll
-    for (int q = 0; q < kAdjGrad; ++q) s[q] = R{};
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += BLOCK)
-#pragma unroll
-        for (int q = 0; q < kAdjGrad; ++q) adj_load_add(s[q], a.partials + (int64_t)kAdjGrad * b + q);
-    block_sum_n<BLOCK>(s, red);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < kAdjGrad; ++q) a.grad[q] = adj_value(s[q]);
-        *a.counter = 0u;
-        __threadfence();
-    }
+    for (int q = 0; q < kAdjGrad; ++q) s[q] = df_of(acc[q]);
+    finish_adjoint<float, BLOCK>(s, red, last, a);
 }
 
 // Sum of the accumulated block slots of a backward sweep: grad[q] =
@@ -432,6 +634,14 @@ static int launch_adjoint_t(const pic_grid *g, const void *pos, const void *neg,
     int rc = score_test(g, &a.score);
     if (rc) return rc;
     const int64_t blocks = adjoint_blocks(g);
+    if constexpr (sizeof(T) == 4) {
+        if (wide_eligible(n, kp, pos, neg, lp_in, ln_in) && wide_eligible(n, kp, lp_out, ln_out, lp_out, ln_out)) {
+            const int64_t want = (a.items / 2 + kWideAdjBlock - 1) / kWideAdjBlock;
+            const int64_t wide = std::min({want, blocks, (int64_t)kWideAdjBlocksPerSm * sm_count()});
+            wide_adjoint_kernel<<<(unsigned)wide, kWideAdjBlock, 0, st>>>(a);
+            return check_launch("wide_adjoint_kernel");
+        }
+    }
     if (flat_index32(n, kp))
         adjoint_step_kernel<T, BLOCK, uint32_t><<<(unsigned)blocks, BLOCK, 0, st>>>(a);
     else

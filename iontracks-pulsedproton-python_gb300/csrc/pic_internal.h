@@ -368,9 +368,11 @@ int launch_adjoint(const pic_grid *g, const void *pos, const void *neg, const vo
                    void *lp_out, void *ln_out, double *grad, void *ws, cudaStream_t st, bool accumulate = false);
 int adjoint_accumulate_begin(const pic_grid *g, void *ws, cudaStream_t st);
 // The streaming adjoint (adjoint_stream.cu): float32 grids with
-// adjoint_variant STREAM, or AUTO and at least kAdjStreamMinCells cells (the
-// grid no longer fits L2 and the flat kernel waits on its neighbour loads).
-constexpr int64_t kAdjStreamMinCells = (int64_t)1 << 24;
+// adjoint_variant STREAM, or AUTO and at least kAdjStreamMinCells cells: below,
+// its items are too few to fill the SMs evenly and the eight-wide kernel is the
+// faster one (330^2 x 406, 44 M cells: 221 us a step against 236), above, the
+// plane ring saves neighbour traffic (608^2 x 406, 151 M: 728 against 718).
+constexpr int64_t kAdjStreamMinCells = 100000000;
 bool adjoint_stream_eligible(const pic_grid *g);
 int launch_adjoint_stream(const pic_grid *g, const void *pos, const void *neg, const void *dens, const void *lp_in,
                           const void *ln_in, void *lp_out, void *ln_out, double *grad, unsigned int *counter,

@@ -108,3 +108,54 @@ def test_arrivals_drawn_in_blocks_equal_numpys(n, bins):
         arrival *= cfg.pulse_duration_s
         assert np.array_equal(got, np.histogram(arrival, edges)[0])
         assert mine.random() == theirs.random()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("wall", [0, 1])
+@pytest.mark.parametrize("n,no_z", SIZES)
+def test_flat_adjoint_step_matches_the_float64_one(n, no_z, wall):
+    """One reverse step against the float64 kernel (which reads the state's
+    neighbours where this one sums by parts). lambda: ten roundings of values
+    within 2 of the peak, 1e-6 of it; each derivative: 1e-6 of the sum of
+    its terms' magnitudes (twelve weights of mu u at most, (1 + mu) p n)."""
+    import ctypes
+
+    import torch
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    lib = native.load()
+    rng = np.random.default_rng(n + no_z)
+    nzb = no_z + 4
+    kp = (nzb + 7) // 8 * 8
+    fields = np.zeros((4, n, n, kp))
+    fields[:2, :, :, 1 : nzb - 1] = rng.uniform(0.5, 1.5, (2, n, n, nzb - 2))
+    fields[2:, :, :, 1 : nzb - 1] = rng.uniform(-1.0, 1.0, (2, n, n, nzb - 2))
+    pairs = rng.uniform(0.0, 1.0, (n, (n + 3) // 4 * 4, 2))
+
+    def step(dtype, dep):
+        t = torch.float64 if dtype == native.PIC_F64 else torch.float32
+        g = _grid(native, n, no_z, wall, dtype, native.PIC_VARIANT_FLAT)
+        g.adjoint_variant = native.PIC_VARIANT_FLAT
+        f = torch.from_numpy(fields).to("cuda", t)
+        out = torch.full((2, n, n, kp), 7.0, dtype=t, device="cuda")
+        d = torch.from_numpy(pairs).to("cuda", t).contiguous()
+        grad = torch.zeros(5, dtype=torch.float64, device="cuda")
+        b = ctypes.c_int64()
+        native.check(lib.pic_adjoint_workspace_bytes(ctypes.byref(g), ctypes.byref(b)), "bytes")
+        ws = torch.zeros(b.value, dtype=torch.uint8, device="cuda")
+        native.check(lib.pic_adjoint_step(ctypes.byref(g), f[0].data_ptr(), f[1].data_ptr(), d.data_ptr() if dep else None,
+                                          f[2].data_ptr(), f[3].data_ptr(), out[0].data_ptr(), out[1].data_ptr(),
+                                          grad.data_ptr(), ws.data_ptr(), ws.numel(),
+                                          torch.cuda.current_stream().cuda_stream), "pic_adjoint_step")
+        return out.double().cpu().numpy(), grad.cpu().numpy()
+
+    for dep in (True, False):
+        lam, grad = step(native.PIC_F32, dep)
+        ref, rgrad = step(native.PIC_F64, dep)
+        assert np.abs(lam - ref).max() <= 1e-6 * max(1.0, np.abs(ref).max())
+        assert not lam[:, :, :, nzb - 1 :].any() and not lam[:, :, :, 0].any()
+        fold = 4 if wall else 1  # a corner column holds its own lambda and three ring columns'
+        mu, u = np.abs(fields[2:]) * fold, fields[:2] + (2.0 if dep else 0.0)
+        sums = [12 * (mu[q] * u[q]).sum() + 4 * mu[q].sum() for q in (0, 0, 1, 1)]
+        sums.append(((1 + mu[0] + mu[1]) * u[0] * u[1]).sum())
+        assert (np.abs(grad - rgrad) <= 1e-6 * np.array(sums)).all()
