@@ -123,6 +123,33 @@ struct Tally<double> {
     __device__ __forceinline__ double value() const { return s; }
 };
 
+// Steps follow one another on a stream, each waiting for all of the one
+// before. launch_linked lets the next launch's blocks be set up while the last
+// blocks of this one finish (programmatic dependent launch): a linked kernel
+// touches memory only behind wait_for_prev(), which returns once every earlier
+// launch is complete and its writes are seen, and calls let_next_start() when
+// its blocks have stepped (earlier, the waiting blocks of the next steps take
+// places unevenly: a float64 step of 24^2 x 206 10.3 us unlinked, 23.5 us with the
+// call first, 7.6 us so). Measured so, us a step, unlinked / linked: float32 30^2 x
+// 406 6.2 / 3.9, 61^2 x 606 10.3 / 8.1, 119^2 x 406 19.4 / 17.9, 208^2 x 406 53.4 /
+// 51.8, 330^2 x 406 124.5 / 123.1; float64 36^2 x 206 with 40 tracks 19.2 / 17.2,
+// 60^2 x 406 63.6 / 61.1.
+__device__ __forceinline__ void wait_for_prev() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline void launch_linked(void (*kernel)(P...), unsigned blocks, int threads, cudaStream_t st, const A &...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);  // (an error is check_launch's to find)
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

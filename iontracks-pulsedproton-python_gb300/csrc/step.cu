@@ -65,12 +65,14 @@ __device__ __forceinline__ bool sums_prev(const StepArgs<T> &a, unsigned &block,
 
 template <typename T, int BLOCK, typename I>
 __global__ void __launch_bounds__(BLOCK) step_kernel(StepArgs<T> a) {
+    wait_for_prev();
     unsigned block, blocks;
     if (sums_prev<T, BLOCK>(a, block, blocks)) return;
     Tally<T> t_rec, t_p, t_n, t_inj;
     const I stride = (I)blocks * BLOCK, items = (I)a.items;
     for (I item = (I)block * BLOCK + threadIdx.x; item < items; item += stride)
         flat_item<T, I>(a, item, t_rec, t_p, t_n, t_inj);
+    let_next_start();
     if (!a.tally) return;  // no tallies wanted (a recomputation): no reduction
     if constexpr (sizeof(T) == 4) {
         DF v[4] = {df_of(t_inj), df_of(t_rec), df_of(t_p), df_of(t_n)};
@@ -84,11 +86,13 @@ __global__ void __launch_bounds__(BLOCK) step_kernel(StepArgs<T> a) {
 // The float32 step over eight-wide items (pic_wide.cuh).
 constexpr int kWideBlock = 256, kWideBlocksPerSm = 2;
 __global__ void __launch_bounds__(kWideBlock, kWideBlocksPerSm) wide_step_kernel(StepArgs<float> a) {
+    wait_for_prev();
     unsigned block, blocks;
     if (sums_prev<float, kWideBlock>(a, block, blocks)) return;
     WideTally tl;
     wide_sweep(a, a.pos_in, a.neg_in, a.pos_out, a.neg_out, a.dens, a.dens_zero, block * kWideBlock + threadIdx.x,
                blocks * kWideBlock, tl);
+    let_next_start();
     if (!a.tally) return;
     DF v[4];
     tl.store(v);
@@ -170,15 +174,15 @@ static int launch_step_t(const pic_grid *g, const void *pos_in, const void *neg_
     }
     if constexpr (sizeof(T) == 4) {
         if (wide) {
-            wide_step_kernel<<<(unsigned)blocks, kWideBlock, 0, st>>>(a);
+            launch_linked(wide_step_kernel, (unsigned)blocks, kWideBlock, st, a);
             return check_launch("wide_step_kernel");
         }
     }
     // (items + stride stays below 2^32 on the 32-bit path: items < 2^29)
     if (flat_index32(g->no_xy, g->kpitch))
-        step_kernel<T, BLOCK, uint32_t><<<(unsigned)blocks, BLOCK, 0, st>>>(a);
+        launch_linked(step_kernel<T, BLOCK, uint32_t>, (unsigned)blocks, BLOCK, st, a);
     else
-        step_kernel<T, BLOCK, int64_t><<<(unsigned)blocks, BLOCK, 0, st>>>(a);
+        launch_linked(step_kernel<T, BLOCK, int64_t>, (unsigned)blocks, BLOCK, st, a);
     return check_launch("step_kernel");
 }
 
