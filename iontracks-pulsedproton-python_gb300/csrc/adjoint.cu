@@ -318,6 +318,7 @@ __global__ void __launch_bounds__(kWideAdjBlock, kWideAdjBlocksPerSm) wide_adjoi
     constexpr int BLOCK = kWideAdjBlock;
     __shared__ DF red[BLOCK / 32][kAdjGrad];
     __shared__ bool last;
+    wait_for_prev();
     Tally2 acc[kAdjGrad];
     const uint32_t n = (uint32_t)a.n, kp = (uint32_t)a.kp, c8 = kp / 8, dp = (uint32_t)a.dp, di = n * kp, w = n - 2;
     const uint32_t inner = w * w, all = n * n, r = blockIdx.x * BLOCK + threadIdx.x, T = gridDim.x * BLOCK;
@@ -485,6 +486,7 @@ __global__ void __launch_bounds__(kWideAdjBlock, kWideAdjBlocksPerSm) wide_adjoi
         }
         if (many) break;
     }
+    let_next_start();
     DF s[kAdjGrad];
 #pragma unroll
     for (int q = 0; q < kAdjGrad; ++q) s[q] = df_of(acc[q]);
@@ -515,6 +517,8 @@ __global__ void __launch_bounds__(BLOCK) adjoint_collect_kernel(const double *sl
 // the ring columns that copy it, so no two threads write the same value.
 template <typename T>
 __global__ void adjoint_fold_kernel(T *lp, T *ln, int64_t n, int64_t kp, int64_t n_edge) {
+    wait_for_prev();
+    let_next_start();
     const int64_t c4 = kp / 4;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n_edge * c4) return;
@@ -588,8 +592,8 @@ static int launch_adjoint_t(const pic_grid *g, const void *pos, const void *neg,
         const int64_t m = n - 2;
         const int64_t n_edge = m + (m > 1 ? m : 0) + (m > 2 ? 2 * (m - 2) : 0);
         const int64_t threads = n_edge * (kp / 4);
-        adjoint_fold_kernel<T><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>((T *)lp_in, (T *)ln_in, n, kp,
-                                                                                 n_edge);
+        launch_linked(adjoint_fold_kernel<T>, (unsigned)((threads + 255) / 256), 256, st, (T *)lp_in, (T *)ln_in, n, kp,
+                      n_edge);
         int rc = check_launch("adjoint_fold_kernel");
         if (rc) return rc;
     }
@@ -638,7 +642,7 @@ static int launch_adjoint_t(const pic_grid *g, const void *pos, const void *neg,
         if (wide_eligible(n, kp, pos, neg, lp_in, ln_in) && wide_eligible(n, kp, lp_out, ln_out, lp_out, ln_out)) {
             const int64_t want = (a.items / 2 + kWideAdjBlock - 1) / kWideAdjBlock;
             const int64_t wide = std::min({want, blocks, (int64_t)kWideAdjBlocksPerSm * sm_count()});
-            wide_adjoint_kernel<<<(unsigned)wide, kWideAdjBlock, 0, st>>>(a);
+            launch_linked(wide_adjoint_kernel, (unsigned)wide, kWideAdjBlock, st, a);
             return check_launch("wide_adjoint_kernel");
         }
     }

@@ -155,6 +155,7 @@ __device__ __forceinline__ void batched_step_block(const BatchStepArgs<T> &b, in
     }
     if constexpr (!COH) {
         // the launches' tallies: batched_tallies_kernel, a group of steps at once
+        let_next_start();
         leave_partial<BLOCK>(v, b.partials + 4 * (int64_t)blk);
         return;
     }
@@ -200,6 +201,7 @@ __global__ void __launch_bounds__(BLOCK, sizeof(T) == 4 ? 4 : 1) batched_step_ke
     // the block's grid arguments, staged once in shared memory and read by
     // broadcast (keeps them out of the registers of every thread)
     __shared__ StepArgs<T> a;
+    wait_for_prev();
     batched_step_block<T, BLOCK, I, false, sizeof(T) == 4 && sizeof(I) == 4>(b, blockIdx.x, red, last, a);
 }
 
@@ -444,7 +446,7 @@ static void launch_batched_step(const BatchLaunch &L, int bi, int bo, double *pa
                        (const T *)L.pos[bi], (const T *)L.neg[bi], (T *)L.pos[bo], (T *)L.neg[bo],
                        (const pair_t<T> *)dens, (pair_t<T> *)dens_zero, L.tally, partials, counters, step,
                        (((uintptr_t)L.pos[0] | (uintptr_t)L.pos[1] | (uintptr_t)L.neg[0] | (uintptr_t)L.neg[1]) & 31) == 0};
-    batched_step_kernel<T, BLOCK, I><<<(unsigned)L.n_blocks, BLOCK, 0, st>>>(b);
+    launch_linked(batched_step_kernel<T, BLOCK, I>, (unsigned)L.n_blocks, BLOCK, st, b);
 }
 
 // ---------------------------------------------------------------------------
