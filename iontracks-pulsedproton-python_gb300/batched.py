@@ -32,7 +32,7 @@ import numpy as np
 
 from . import _native as N
 from .config import SimulationConfig
-from .engine import make_grid, nvtx_range
+from .engine import make_grid, nvtx_range, runs_resident
 from .feeder import TrackFeeder
 from .pulses import TrackSampler, build_track_schedule
 from .state import Diagnostics, collection_efficiency
@@ -54,6 +54,36 @@ MAX_ITEMS_PER_BLOCK = 1 << 16
 # there the batched launch is bound by its per-block table and reduction work
 # (23 us a step for one 53 x 53 x 208 grid), the flat step kernel is not.
 SOLO_MAX_GRIDS = 2
+
+
+def _solo_us(cells: float, resident: bool) -> float:
+    """Microseconds a step of one float32 grid of ``cells`` million cells takes
+    alone: resident 24^2 x 206 2.1, 53^2 x 206 3.0, 59^2 x 406 5.5; flat 30^2 x 406
+    3.9, 61^2 x 606 8.1, 119^2 x 406 17.9, 208^2 x 406 (past the L2) 51.8."""
+    return 1.7 + 2.6 * cells if resident else max(3.0 + 2.5 * cells, 2.9 * cells)
+
+
+def _batched_us(cells: float) -> float:
+    """Microseconds of a batched step over ``cells`` million cells: 4.3 M 24.0, 8.1 M
+    37.6, 10.4 M 48.7 (every grid a step at a time, the fields pass through
+    the L2), 48.7 M 178."""
+    return 5.0 + 4.3 * min(cells, 10.5) + 3.3 * max(0.0, cells - 10.5)
+
+
+def solo_from(phases, cells, resident) -> int:
+    """The first phase (of ``_phases``) from which on each phase's grids step one
+    after the other, chunk by chunk, in less than nine tenths of the batched
+    step's time: a chunk of a grid alone keeps its fields in the L2 or on the
+    chip. ``cells[c]``: million cells of grid c, ``resident[c]``: it runs
+    resident. Phases before it are not (the pairs a grid stepped alone leaves
+    are not what the batched step expects). Three grids of 8.1 M cells: 37.6 us
+    a step batched, 28 one after the other."""
+    first = len(phases)
+    for _, _, active in reversed(phases):
+        if sum(_solo_us(cells[c], resident[c]) for c in active) >= 0.9 * _batched_us(sum(cells[c] for c in active)):
+            break
+        first -= 1
+    return first
 
 
 # The streaming batched step (pic_batched_stream_*): 15 consumer warps of up to
@@ -412,7 +442,8 @@ def run_batched_b200(
     64-configuration sweep the per-step launches are faster (1.31 vs 1.44 s):
     two device-wide barriers per step cost what two launch gaps do.
     Phases with at most ``solo_grids`` active grids run each grid's chunk
-    with the single-grid kernels instead (0: never). ``variant`` picks the
+    with the single-grid kernels instead, and so do the last phases of float32
+    batches where that is the faster way (``solo_from``; 0: never). ``variant`` picks the
     fused step of the batched launches: "flat" (pic_batched_segment, neighbours
     through L1/L2), "stream" (pic_batched_stream_segment: float32, planes staged
     in a shared-memory ring, items from every grid taken from a device-wide
@@ -550,11 +581,17 @@ def run_batched_b200(
     # --- work tables, one per set of active grids
     phases = []
     max_blocks = 1
-    for s0, s1, active in _phases(totals):
+    plain = _phases(totals)
+    solo_first = len(plain)
+    if solo_grids > 0 and dtype == "float32" and not persistent and variant != "stream":
+        solo_first = solo_from(plain, [int(g.no_xy) ** 2 * int(g.nzb) * 1e-6 for g in grids],
+                               [runs_resident(g) for g in grids])
+    for k, (s0, s1, active) in enumerate(plain):
         wt = _work_table(items, active, sms)
         max_blocks = max(max_blocks, len(wt["blk_cfg"]))
         phases.append((s0, s1, dict(
             active=[int(c) for c in active],
+            solo=not persistent and solo_grids > 0 and (len(active) <= solo_grids or k >= solo_first),
             n_blocks=int(len(wt["blk_cfg"])),
             **{k: torch.from_numpy(v).to(dev) for k, v in wt.items()},
         )))
@@ -569,7 +606,7 @@ def run_batched_b200(
     if variant in ("stream", "mixed") and dtype == "float32" and not persistent:
         shapes = [(int(g.no_xy), int(g.nzb), int(g.kpitch)) for g in grids]
         for s0, _, tab in phases:
-            if solo_grids > 0 and len(tab["active"]) <= solo_grids:
+            if tab["solo"]:
                 continue
             if not stream_phase(shapes, tab["active"], variant, dtype, persistent):
                 continue
@@ -584,7 +621,7 @@ def run_batched_b200(
                                                    sws.numel(), st, ctypes.byref(bs)), "pic_batched_stream_prepare")
             stream_tabs[s0] = (bs, sws)
     solo_ws = None
-    if solo_grids > 0 and not persistent and any(len(t["active"]) <= solo_grids for _, _, t in phases):
+    if any(t["solo"] for _, _, t in phases):
         need = 0
         for g in grids:  # one workspace for every solo grid: the largest any of them needs
             swb = ctypes.c_int64()
@@ -675,7 +712,7 @@ def run_batched_b200(
             feeder.upload(pending, xs_dev, ys_dev)
             # draw the next chunk's tracks while the device runs this one
             pending = feeder.submit(jobs_of(*chunks[k + 1][:2])) if k + 1 < len(chunks) else None
-            if solo_ws is not None and len(tab["active"]) <= solo_grids:
+            if tab["solo"]:
                 with nvtx_range(f"solo grids ({len(tab['active'])})"):
                     for c in tab["active"]:  # independent grids: one after the other
                         run_solo(c, c0, c1)

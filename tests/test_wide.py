@@ -159,3 +159,23 @@ def test_flat_adjoint_step_matches_the_float64_one(n, no_z, wall):
         sums = [12 * (mu[q] * u[q]).sum() + 4 * mu[q].sum() for q in (0, 0, 1, 1)]
         sums.append(((1 + mu[0] + mu[1]) * u[0] * u[1]).sum())
         assert (np.abs(grad - rgrad) <= 1e-6 * np.array(sums)).all()
+
+
+@pytest.mark.parametrize("seed", range(5))
+def test_grids_step_alone_from_a_phase_on(seed):
+    """The phases a batch steps grid by grid are the last ones: all those, and no
+    more, from which on every phase is estimated faster so."""
+    batched = importlib.import_module(pkg().__name__ + ".batched")
+    rng = np.random.default_rng(seed)
+    cells = rng.choice([0.1, 0.5, 2.0, 6.0, 20.0, 60.0], 12)
+    resident = cells < 1.0
+    phases = batched._phases(rng.integers(1, 40, 12))
+
+    def alone(active):
+        own = sum(batched._solo_us(cells[c], resident[c]) for c in active)
+        return own < 0.9 * batched._batched_us(sum(cells[c] for c in active))
+
+    first = batched.solo_from(phases, cells, resident)
+    assert all(alone(active) for _, _, active in phases[first:])
+    assert first == 0 or not alone(phases[first - 1][2])
+    assert batched.solo_from([], [], []) == 0
