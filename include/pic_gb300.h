@@ -76,7 +76,7 @@ typedef struct pic_grid {
     /* Adjoint step kernel (pic_adjoint_*, pic_revolve_backward): a
      * PIC_VARIANT_* of its own, so tuning the step's shape leaves it alone.
      * AUTO: STREAM for float32 grids with no_xy >= 4 and no_xy^2 * kpitch >=
-     * 2^24 cells, FLAT otherwise; STREAM on a float64 grid is refused. */
+     * 1e8 cells, FLAT otherwise; STREAM on a float64 grid is refused. */
     int32_t adjoint_variant;
     /* Deposition form (PIC_DEPOSIT_*). */
     int32_t deposit_variant;
@@ -105,11 +105,11 @@ typedef struct pic_grid {
 #define PIC_DEPOSIT_TRACKS 1
 #define PIC_DEPOSIT_BINNED 2
 
-/* Fused-step kernels. FLAT: one thread per four k of a column, neighbours
+/* Fused-step kernels. FLAT: one thread per eight k of a column (float64: four), neighbours
  * through L1/L2, any grid and either field type. STREAM: float32 only; whole
  * (j-tile x k-row) planes staged in shared memory by bulk asynchronous copies
  * while the CTA marches along i, for grids with no_xy >= 16. AUTO picks
- * STREAM for float32 grids with no_xy >= 64 and no_xy^2 * kpitch >= 1e8 cells,
+ * STREAM for float32 grids with no_xy >= 64 and no_xy^2 * kpitch >= 2e8 cells,
  * FLAT otherwise, and segments of small float32 grids run resident
  * (pic_segment_resident); planes_per_item 0 gives about 12 work items per SM,
  * consumer_warps 0 gives 13, tile_rows 0 about three k-vectors a consumer

@@ -101,12 +101,11 @@ int score_test(const pic_grid *g, ScoreTest *out) {
 }
 
 int resolve_shape(pic_grid *g) {
-    // Measured on GB300 (graph-replayed steps, idle / pulse): the flat kernel
-    // is faster up to a few hundred lateral cells (62.6 / 77.9 us vs 86.4 /
-    // 95.8 us at 208x208x408; 146 / 174 vs 176 / 191 us at 328x328x408); the
-    // streaming kernel in its 13-consumer-warp form wins from 608x608x408
-    // (437 / 438 vs 454 / 492 us) to the 1068x1068x408 full electrode (1.250 /
-    // 1.255 ms vs 1.73 / 1.95 ms).
+    // Measured on GB300 (us a step of a segment, idle / 1500 tracks, flat
+    // against streaming in its 13-consumer-warp form): 330^2 x 406 123 / - vs
+    // 156 / -, 536^2 x 406 317 / 325 vs 347 / 352, 680^2 x 406 (189 M cells) 515 / 525
+    // vs 527 / 535, 740^2 x 406 (223 M) 607 / 617 vs 605 / 611, 1068^2 x 406 1320 vs
+    // 1195.
     if (g->variant == PIC_VARIANT_AUTO)
         g->variant = (g->dtype == PIC_F32 && g->no_xy >= 64 && g->no_xy * g->no_xy * g->kpitch >= kStreamMinCells)
                          ? PIC_VARIANT_STREAM
