@@ -179,3 +179,15 @@ def test_grids_step_alone_from_a_phase_on(seed):
     assert all(alone(active) for _, _, active in phases[first:])
     assert first == 0 or not alone(phases[first - 1][2])
     assert batched.solo_from([], [], []) == 0
+
+
+@pytest.mark.parametrize("n,no_z,wall,expected", [(51, 600, 0, 0), (51, 600, 1, 1), (59, 400, 0, 1), (86, 200, 0, 1)])
+def test_tall_absorbing_grids_step_flat(n, no_z, wall, expected):
+    """Grids whose resident division is estimated slower than the flat step."""
+    import ctypes
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    out = ctypes.c_int32(-1)
+    g = _grid(native, n, no_z, wall, native.PIC_F32, 0)
+    native.check(native.load().pic_segment_resident(ctypes.byref(g), ctypes.byref(out)), "pic_segment_resident")
+    assert out.value == expected
