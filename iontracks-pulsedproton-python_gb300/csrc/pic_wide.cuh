@@ -17,7 +17,10 @@
 // a segment without tracks, four-wide / here (the tallies' share in pic_internal.h):
 // 30^2 x 406 9.6 / 6.2, 61^2 x 606 14.4 / 10.3, 119^2 x 406 26.0 / 19.6, 208^2 x 406
 // 60.5 / 53.3, 330^2 x 406 137.5 / 124.2, 608^2 x 406 449 / 412; with 1500 tracks a
-// step, their deposition included, 208^2 x 406 68.9 / 59.0.
+// step, their deposition included, 208^2 x 406 68.9 / 59.0. With linked launches
+// (pic_device.cuh), absorbing / reflecting wall: 51^2 x 606 6.6 / 6.7, 119^2 x 406 17.3 /
+// 17.8, 208^2 x 406 50.8 / 51.4, 330^2 x 406 121 absorbing (the reflecting ring's
+// writes as a loop over its eight sides: 6.7 / 7.5, 17.6 / 18.9, 51.2 / 52.0).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -233,15 +236,22 @@ __device__ __forceinline__ void wide_sweep(const StepArgs<float> &a, const float
                 store8(pos_out + base, LP);
                 store8(neg_out + base, LN);
                 if (k0 == 0 && dens_zero) dens_zero[dcol] = float2{0.f, 0.f};
-                if (a.reflecting && (i == 1 || i == w || j == 1 || j == w)) {
+                if (a.reflecting) {
                     // the ring columns whose nearest interior column this is
-#pragma unroll 1
-                    for (int e = 0; e < 9; ++e) {
-                        const int si = e / 3 - 1, sj = e % 3 - 1;
-                        if (e == 4 || (si && i != (si < 0 ? 1 : w)) || (sj && j != (sj < 0 ? 1 : w))) continue;
-                        const uint32_t o = base + (uint32_t)si * di + (uint32_t)sj * kp;
+                    const bool up = i == 1, down = i == w, left = j == 1, right = j == w;
+                    auto ring = [&](uint32_t o) {
                         store8(pos_out + o, LP);
                         store8(neg_out + o, LN);
+                    };
+                    if (up) ring(base - di);
+                    if (down) ring(base + di);
+                    if (left || right) {
+                        if (left) ring(base - kp);
+                        if (right) ring(base + kp);
+                        if (up && left) ring(base - di - kp);
+                        if (up && right) ring(base - di + kp);
+                        if (down && left) ring(base + di - kp);
+                        if (down && right) ring(base + di + kp);
                     }
                 }
                 v += step;
@@ -251,6 +261,7 @@ __device__ __forceinline__ void wide_sweep(const StepArgs<float> &a, const float
                 if (j > w) j -= w, ++i, at += 2 * kp;
             }
         }
+        if (a.reflecting && !dens_zero) v = all;
         for (; v < all; v += step) {
             const uint32_t u = v - inner;  // ring: row 0, row n-1, then the two ends of each row between
             if (u < 2 * n) i = u < n ? 0 : n - 1, j = u < n ? u : u - n;

@@ -564,19 +564,18 @@ bool ResPlanMemo::plan(const pic_grid *g, const ResPatch *patches, int count, Re
     return fits;
 }
 
-// Estimated microseconds of a flat step of an absorbing grid that stays in the L2
-// (pic_wide.cuh): 30^2 x 406 3.9, 61^2 x 606 8.1, 119^2 x 406 17.9.
+// Estimated microseconds of a flat step of a grid that stays in the L2
+// (pic_wide.cuh): 30^2 x 406 3.9, 61^2 x 606 8.1, 119^2 x 406 17.4.
 static double flat_cost(const pic_grid *g) { return 3.0 + 2.5e-6 * (double)(g->no_xy * g->no_xy * g->nzb); }
 
-// Absorbing grids whose division is estimated slower than the flat step run flat:
-// few and tall columns, which the SMs split badly (51^2 x 606: resident 12.6 ms for
-// 1500 steps, flat 11.5; estimates 7.9 and 6.9 us a step; 61^2 x 406 the same either
-// way, 86^2 x 206 11.5 against 12.1). A reflecting wall's flat step writes the ring
-// besides and is the slower one there too (13.2 against 12.1 ms).
+// Grids whose division is estimated slower than the flat step run flat: few and
+// tall columns, which the SMs split badly (51^2 x 606, ms for 1500 steps, absorbing /
+// reflecting: resident 12.6 / 12.3, flat 11.4 / 12.0; estimates 7.9 and 6.9 us a step.
+// 61^2 x 406 the same either way, 86^2 x 206 11.5 resident, 12.1 flat).
 bool resident_plan(const pic_grid *g, ResPlan *out) {
     static thread_local ResPlanMemo memo;
     if (!memo.plan(g, kPatches, (int)(sizeof(kPatches) / sizeof(kPatches[0])), step_smem, 1.0, out)) return false;
-    return g->wall == PIC_WALL_REFLECTING || plan_cost(*out, kPatches[out->patch], 1.0) <= flat_cost(g);
+    return plan_cost(*out, kPatches[out->patch], 1.0) <= flat_cost(g);
 }
 
 int launch_resident(const pic_grid *g, const ResPlan &p, const void *pos_in, const void *neg_in, void *pos_out,

@@ -181,8 +181,8 @@ def test_grids_step_alone_from_a_phase_on(seed):
     assert batched.solo_from([], [], []) == 0
 
 
-@pytest.mark.parametrize("n,no_z,wall,expected", [(51, 600, 0, 0), (51, 600, 1, 1), (59, 400, 0, 1), (86, 200, 0, 1)])
-def test_tall_absorbing_grids_step_flat(n, no_z, wall, expected):
+@pytest.mark.parametrize("n,no_z,wall,expected", [(51, 600, 0, 0), (51, 600, 1, 0), (59, 400, 0, 1), (86, 200, 0, 1)])
+def test_tall_grids_step_flat(n, no_z, wall, expected):
     """Grids whose resident division is estimated slower than the flat step."""
     import ctypes
 
