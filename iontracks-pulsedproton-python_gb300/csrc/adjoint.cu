@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kWideAdjBlock, kWideAdjBlocksPerSm) wide_adjoi
             const bool act = v < inner;
             const uint32_t base = act ? at : n * kp + kp + (uint32_t)k0;
             float2 d = {0.f, 0.f};
-            if (a.dens) d = __ldg(a.dens + (act ? i * dp + j : dp + 1));
+            if (a.dens) d = a.dens[act ? i * dp + j : dp + 1];
             const Oct MP = load8(a.lp + base), MN = load8(a.ln + base);
             Oct LP = zero8(), LN = zero8();
             {
@@ -376,8 +376,8 @@ __global__ void __launch_bounds__(kWideAdjBlock, kWideAdjBlocksPerSm) wide_adjoi
             const Oct P = load8(a.pos + base), N = load8(a.neg + base);
             float ep = 0.f, en = 0.f;
             if (edge_lane) {
-                ep = __ldg(a.lp + (base + edge_off));
-                en = __ldg(a.ln + (base + edge_off));
+                ep = a.lp[base + edge_off];
+                en = a.ln[base + edge_off];
             }
             // (mu is zero on a column's end layers and padding, so the value
             // of a lane that holds another column's end is right here)

@@ -29,25 +29,27 @@ __host__ __device__ inline T centre_weight(double lat, double zm, double zp, dou
 // Four consecutive k elements of one (i, j) column. The field rows are
 // 32-byte aligned (kpitch is a multiple of 8) and every vector starts at a
 // multiple of 4 elements, so float loads are single 128-bit accesses and
-// double loads two 128-bit accesses.
+// double loads two 128-bit accesses. Plain loads: the read-only path (__ldg) is
+// for data that nothing writes during the kernel's life, and a linked kernel
+// (below) is resident while the launch before it writes what it reads.
 template <typename T>
 struct V4 {
     T v[4];
 };
 
 __device__ __forceinline__ V4<float> load4(const float *p) {
-    float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+    const float4 t = *reinterpret_cast<const float4 *>(p);
     return {{t.x, t.y, t.z, t.w}};
 }
 __device__ __forceinline__ V4<double> load4(const double *p) {
-    double2 a = __ldg(reinterpret_cast<const double2 *>(p));
-    double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
+    const double2 a = *reinterpret_cast<const double2 *>(p);
+    const double2 b = *(reinterpret_cast<const double2 *>(p) + 1);
     return {{a.x, a.y, b.x, b.y}};
 }
 // Coherent forms for kernels that read data written earlier in the same
 // launch by other blocks (the persistent kernels): loads cached in L2 only
-// (ld.global.cg). Neither the read-only path of __ldg nor an SM's L1 is kept
-// coherent with other SMs' writes; L2 is the point of coherence.
+// (ld.global.cg). An SM's L1 is not kept coherent with other SMs' writes; L2 is
+// the point of coherence.
 __device__ __forceinline__ V4<float> load4c(const float *p) {
     const float4 t = __ldcg(reinterpret_cast<const float4 *>(p));
     return {{t.x, t.y, t.z, t.w}};
@@ -127,7 +129,8 @@ struct Tally<double> {
 // before. launch_linked lets the next launch's blocks be set up while the last
 // blocks of this one finish (programmatic dependent launch): a linked kernel
 // touches memory only behind wait_for_prev(), which returns once every earlier
-// launch is complete and its writes are seen, and calls let_next_start() when
+// launch is complete and its writes are seen by coherent loads (not by the
+// read-only path: none in such a kernel), and calls let_next_start() when
 // its blocks have stepped (earlier, the waiting blocks of the next steps take
 // places unevenly: a float64 step of 24^2 x 206 10.3 us unlinked, 23.5 us with the
 // call first, 7.6 us so). Measured so, us a step, unlinked / linked: float32 30^2 x

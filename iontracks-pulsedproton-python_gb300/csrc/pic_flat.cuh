@@ -68,8 +68,8 @@ __device__ __forceinline__ bool scored_col_t(const ScoreTest &t, I i, I j) {
 // (i, j), decoded from the flat item index (k-vector fastest). Adds the
 // item's scored contributions to the thread's running tallies. I is the index
 // type (uint32_t when flat_index32 holds for the grid, else int64_t). COH:
-// plain (coherent) vector loads instead of the read-only path, for a kernel
-// that reads fields other blocks wrote earlier in the same launch.
+// loads from L2 only, for a kernel that reads fields other blocks wrote earlier
+// in the same launch.
 template <typename T, typename I, bool COH = false>
 __device__ __forceinline__ void flat_item(const StepArgs<T> &a, I item, Tally<T> &t_rec,
                                           Tally<T> &t_p, Tally<T> &t_n, Tally<T> &t_inj) {

@@ -42,12 +42,16 @@ struct Oct {
     float2 v[4];  // eight consecutive k
 };
 
+// (volatile and coherent: a linked kernel, pic_device.cuh, is resident while its
+// input is written, so no load of it may move above wait_for_prev() or take the
+// read-only path)
 __device__ __forceinline__ Oct load8(const float *p) {
     Oct o;
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(o.v[0].x), "=f"(o.v[0].y), "=f"(o.v[1].x), "=f"(o.v[1].y), "=f"(o.v[2].x), "=f"(o.v[2].y),
           "=f"(o.v[3].x), "=f"(o.v[3].y)
-        : "l"(p));
+        : "l"(p)
+        : "memory");
     return o;
 }
 __device__ __forceinline__ void store8(float *p, const Oct &o) {
@@ -155,7 +159,7 @@ __device__ __forceinline__ void wide_sweep(const StepArgs<float> &a, const float
             const uint32_t base = act ? at : n * kp + kp + (uint32_t)k0;  // (column (1, 1) for a lane without one)
             const uint32_t dcol = act ? i * dp + j : dp + 1;
             float2 d = {0.f, 0.f};
-            if (dens) d = __ldg(dens + dcol);  // (in flight with the fields)
+            if (dens) d = dens[dcol];  // (in flight with the fields)
             Oct P = load8(pos_in + base), N = load8(neg_in + base);
             const Oct Pim = load8(pos_in + (base - di)), Pip = load8(pos_in + (base + di));
             const Oct Pjm = load8(pos_in + (base - kp)), Pjp = load8(pos_in + (base + kp));
@@ -163,8 +167,8 @@ __device__ __forceinline__ void wide_sweep(const StepArgs<float> &a, const float
             const Oct Njm = load8(neg_in + (base - kp)), Njp = load8(neg_in + (base + kp));
             float ep = 0.f, en = 0.f;
             if (edge_lane) {
-                ep = __ldg(pos_in + (base + edge_off));
-                en = __ldg(neg_in + (base + edge_off));
+                ep = pos_in[base + edge_off];
+                en = neg_in[base + edge_off];
             }
             Oct LP, LN;
 #pragma unroll
@@ -270,7 +274,7 @@ __device__ __forceinline__ void wide_sweep(const StepArgs<float> &a, const float
                 const uint32_t o = (i * n + j) * kp + (uint32_t)k0;
                 Oct P = load8(pos_in + o), N = load8(neg_in + o);
                 if (dens) {
-                    const float d = __ldg(dens + (i * dp + j)).x;
+                    const float d = dens[i * dp + j].x;
                     const uint32_t m[8] = {spread<0>(g_lo), spread<1>(g_lo), spread<2>(g_lo), spread<3>(g_lo),
                                            spread<0>(g_hi), spread<1>(g_hi), spread<2>(g_hi), spread<3>(g_hi)};
 #pragma unroll
