@@ -159,7 +159,7 @@ int pic_segment_workspace_bytes(const pic_grid *g, int64_t *bytes);
  * library's choice for float32 grids of up to about a million cells with
  * variant AUTO, steps_per_launch 0, a deposit_variant other than TRACKS and
  * cutoff_voxels < 31.5 (segments of at least 4 steps, 65536 tracks a step at
- * most); else 0. A segment of a few launches gains nothing from a CUDA graph. */
+ * most, none so dense that depositing step by step is faster); else 0. A segment of a few launches gains nothing from a CUDA graph. */
 int pic_segment_resident(const pic_grid *g, int32_t *resident);
 
 /* Reads (and with reset != 0 clears) the status word a kernel sets in the

@@ -240,7 +240,7 @@ static int run_loop(const pic_grid *g, void *pos0, void *neg0, void *pos1, void 
         return PIC_OK;
     }
     ResPlan plan;
-    if (resident_steps_eligible(g, ws, ws_bytes, off, n_steps, &plan)) {
+    if (resident_steps_eligible(g, ws, ws_bytes, off, n_steps, n_steps, &plan)) {
         const void *last_pairs = nullptr;
         int bi = (int)(parity & 1);
         for (int64_t s0 = 0; s0 < n_steps;) {
@@ -597,7 +597,8 @@ int pic_adjoint_forward(const pic_grid *g, void *pos0, void *neg0, void *pos1, v
         return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaMemcpyAsync(checkpoint)", e);
     };
     ResPlan plan;
-    if (ckpt_every >= kResMinSteps && resident_steps_eligible(g, workspace, workspace_bytes, track_offsets, n_steps, &plan)) {
+    if (ckpt_every >= kResMinSteps &&
+        resident_steps_eligible(g, workspace, workspace_bytes, track_offsets, n_steps, ckpt_every, &plan)) {
         // launches up to the next checkpoint, pairs straight into the kept slots
         const void *last_pairs = nullptr;
         int64_t d = 0;

@@ -293,6 +293,12 @@ int64_t next_deposit_group(const int64_t *off, int64_t s0, int64_t n_steps, int 
     return s1;
 }
 
+double bin_tile_tracks(const pic_grid *g, int64_t most) {
+    const int64_t tiles = bin_tiles_per_side(g->no_xy) * bin_tiles_per_side(g->no_xy);
+    const double per_axis = (2.0 * g->cutoff_voxels + kBinC) / kBinOut;  // tiles a track meets along an axis
+    return (double)most * per_axis * per_axis / (double)tiles;
+}
+
 bool deposit_binned(const pic_grid *g, const void *ws, int64_t ws_bytes, int64_t most) {
     const int64_t bin_bytes = dep_bin_bytes(g);
     const bool bins = ws && bin_bytes > 0 && ws_bytes >= kWorkspaceBytes + bin_bytes;
@@ -301,8 +307,7 @@ bool deposit_binned(const pic_grid *g, const void *ws, int64_t ws_bytes, int64_t
     const int64_t tiles = bin_tiles_per_side(g->no_xy) * bin_tiles_per_side(g->no_xy);
     if (most < 0) return tiles >= (int64_t)kBinAutoTilesPerSm * sm_count();  // one step alone
     // grouped: enough blocks for the SMs, or tiles short enough for one block
-    const double per_axis = (2.0 * g->cutoff_voxels + kBinC) / kBinOut;  // tiles a track meets along an axis
-    return tiles * kBinSteps >= sm_count() || (double)most * per_axis * per_axis / (double)tiles <= kBinAutoPerTile;
+    return tiles * kBinSteps >= sm_count() || bin_tile_tracks(g, most) <= kBinAutoPerTile;
 }
 
 // Track-tile pairs a step's deposition may scan in the tile form: beyond it

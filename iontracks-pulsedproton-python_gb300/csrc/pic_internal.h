@@ -290,11 +290,21 @@ inline ResSpace resident_space(const pic_grid *g, const ResPlan &p) {
 inline bool resident_wanted(const pic_grid *g) {
     return g->variant == PIC_VARIANT_AUTO && g->steps_per_launch == 0 && g->deposit_variant != PIC_DEPOSIT_TRACKS;
 }
-// Whether a segment of these steps runs resident: the library's own choice of
-// kernels (no variant, steps per launch or per-track deposition asked for), a
-// workspace of pic_step_workspace_bytes, and tracks the binned deposition takes.
+// Whether a segment of these steps, in launches that end at every span-th,
+// runs resident: the library's own choice of kernels (no variant, steps per
+// launch or per-track deposition asked for), a workspace of
+// pic_segment_workspace_bytes, and tracks the binned deposition takes and is no
+// slower with. It deposits a launch's steps together, a block a step and tile, so
+// it lasts as long as the tile with the most tracks: 80 to 110 ns a track; the
+// per-track warps of the steps launched one by one take 5 us and 5 to 16 ns a
+// track, one step after the other. So a tile's share is to be at most
+// kBinAutoPerTile, as in the flat steps' groups, or, over the launches where it
+// is more, a tenth of their tracks. Measured, us a step of 64, its deposition alone, binned / per track:
+// 24^2 x 206 with 2000 tracks a step 6.6 / 31, 4000 23 / 66, 12000 141 / 139, 20000
+// 383 / 206, 65000 3468 / 579; 18^2 x 56 with 4000 23 / 28, 8000 61 / 50, 20000 382
+// / 109; four steps of 2000 tracks on 48^2 x 206 41 / 23.
 bool resident_steps_eligible(const pic_grid *g, const void *ws, int64_t ws_bytes, const int64_t *off, int64_t n_steps,
-                             ResPlan *plan);
+                             int64_t span, ResPlan *plan);
 // The end of the next resident launch's steps from s0 (at most kResSteps of
 // them and kBinTracks tracks).
 int64_t next_resident_group(const int64_t *off, int64_t s0, int64_t n_steps);
@@ -313,6 +323,8 @@ int launch_deposit_slots(const pic_grid *g, const double *xs, const double *ys, 
                          int64_t s1, uint32_t *hist, void *ws, int64_t counts, int64_t lists, void *dens,
                          int64_t dens_stride, int16_t *slot, cudaStream_t st);
 
+// Of a step's `most` tracks, those a tile of the binned form meets on average.
+double bin_tile_tracks(const pic_grid *g, int64_t most);
 // Whether the deposition takes the binned form for this grid and workspace:
 // for a segment's steps together (most = the most tracks one of them has),
 // or with most < 0 for one step alone.

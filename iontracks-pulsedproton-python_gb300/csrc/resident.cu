@@ -617,12 +617,23 @@ int launch_resident(const pic_grid *g, const ResPlan &p, const void *pos_in, con
 }
 
 bool resident_steps_eligible(const pic_grid *g, const void *ws, int64_t ws_bytes, const int64_t *off, int64_t n_steps,
-                             ResPlan *plan) {
+                             int64_t span, ResPlan *plan) {
     if (!resident_wanted(g) || n_steps < kResMinSteps || !ws || !resident_plan(g, plan) || ws_bytes < resident_space(g, *plan).end)
         return false;
-    int64_t most = 0;
-    for (int64_t s = 0; s < n_steps; ++s) most = std::max(most, off[s + 1] - off[s]);
-    return most == 0 || (most <= kBinTracks && bin_eligible(g));
+    if (off[n_steps] == off[0]) return true;
+    if (!bin_eligible(g)) return false;
+    double longest = 0.0, tracks = 0.0;  // of the launches with a tile of more than kBinAutoPerTile: its tracks, all tracks
+    for (int64_t s0 = 0, s1; s0 < n_steps; s0 = s1) {
+        s1 = next_resident_group(off, s0, std::min(n_steps, (s0 / span + 1) * span));
+        if (s1 == s0) return false;  // a step of more than kBinTracks
+        int64_t most = 0;
+        for (int64_t s = s0; s < s1; ++s) most = std::max(most, off[s + 1] - off[s]);
+        const double tile = bin_tile_tracks(g, most);
+        if (tile <= kBinAutoPerTile) continue;
+        longest += std::min(tile, (double)most);
+        tracks += (double)(off[s1] - off[s0]);
+    }
+    return g->deposit_variant == PIC_DEPOSIT_BINNED || 10.0 * longest <= tracks;
 }
 
 int64_t next_resident_group(const int64_t *off, int64_t s0, int64_t n_steps) {

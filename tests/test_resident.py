@@ -230,3 +230,36 @@ def test_resident_reverse_sweep_matches_the_float64_one(n, no_z, wall):
     voxels = steps * (n - 2) ** 2 * (no_z + 2)
     magnitude = np.array([np.abs(ref).mean() * 2.0] * 4 + [1.0 + np.abs(ref).mean() * 2.0]) * voxels
     assert (np.abs(grad - want) <= 2 * tol * magnitude).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,no_z,tracks,steps,flat", [(24, 100, 600, 4, False), (24, 100, 2000, 4, True), (24, 100, 2000, 16, False),
+                                                      (18, 50, 20000, 12, True), (31, 60, 60000, 5, True)])
+def test_dense_segments_step_flat(n, no_z, tracks, steps, flat):
+    """Steps of so many tracks that one block's sum of them would outlast the
+    per-track deposition of all (resident_steps_eligible): launched one by one."""
+    import torch
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    rng = np.random.default_rng(n + tracks)
+    state = _case(n, no_z, steps, n, 1)[0]
+    off = np.arange(steps + 1, dtype=np.int64) * tracks
+    off[2:] -= tracks  # the second step has none
+    xs, ys = rng.uniform(0, n, (2, off[-1]))
+    g = _grid(native, n, no_z, 0, native.PIC_F32, 0)
+    g64 = _grid(native, n, no_z, 0, native.PIC_F64, 1)
+    g.gaussian_factor = g64.gaussian_factor = 3.0 / tracks
+    before = native.load().pic_kernel_launches()
+    got = _segment(native, g, torch, state, xs, ys, off, 0)
+    launches = native.load().pic_kernel_launches() - before
+    assert launches == (2 * steps - 1 if flat else 4)  # a deposition and a step each; binning, tiles, steps, tallies
+    ref = _segment(native, g64, torch, state, xs, ys, off, 0)
+    # a cell's float32 sum of `tracks` terms of one sign, rounded at each: at
+    # worst half an ulp of the sum a term, and of that a random walk's share,
+    # sqrt(tracks) 3e-8 of the deposition's peak (1.5 at most) with four deviations
+    tol = 1e-6 * steps + 1.5 * 4 * tracks**0.5 * 3e-8 * steps
+    for a, b in zip(got[:2], ref[:2]):
+        assert np.abs(a - b).max() <= tol * np.abs(b).max()
+    for q in range(4):
+        assert np.abs(got[3][:, q] - ref[3][:, q]).max() <= tol * np.abs(ref[3][:, q]).max() + 1e-30
+    assert np.array_equal(got[4], ref[4])
