@@ -131,7 +131,7 @@ struct Tally<double> {
 // touches memory only behind wait_for_prev(), which returns once every earlier
 // launch is complete and its writes are seen by coherent loads (not by the
 // read-only path: none in such a kernel), and calls let_next_start() when
-// its blocks have stepped (earlier, the waiting blocks of the next steps take
+// its blocks have stepped, one that finishes its own tallies as it ends (step.cu; earlier, the waiting blocks of the next steps take
 // places unevenly: a float64 step of 24^2 x 206 10.3 us unlinked, 23.5 us with the
 // call first, 7.6 us so). Measured so, us a step, unlinked / linked: float32 30^2 x
 // 406 6.2 / 3.9, 61^2 x 606 10.3 / 8.1, 119^2 x 406 19.4 / 17.9, 208^2 x 406 53.4 /

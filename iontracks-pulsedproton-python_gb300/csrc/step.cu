@@ -34,6 +34,15 @@
 
 namespace pic {
 
+// Whether the launch finishes its own tallies. It then lets the next one start
+// only as it ends: that one's blocks, waiting on the SMs, slow the chain of its
+// blocks and its last block's sum (float64 lone steps, us, started early / at the
+// end: 24^2 x 206 18.3 / 14.7, 36^2 x 206 28.0 / 22.9; float32 59^2 x 406 10.1 / 9.7).
+template <typename T>
+__device__ __forceinline__ bool finishes(const StepArgs<T> &a) {
+    return a.tally && a.counter;
+}
+
 // The end of a step: the tallies finished here, or (no counter) the block's
 // partials left for the next step's block 0.
 template <int BLOCK>
@@ -72,7 +81,7 @@ __global__ void __launch_bounds__(BLOCK) step_kernel(StepArgs<T> a) {
     const I stride = (I)blocks * BLOCK, items = (I)a.items;
     for (I item = (I)block * BLOCK + threadIdx.x; item < items; item += stride)
         flat_item<T, I>(a, item, t_rec, t_p, t_n, t_inj);
-    let_next_start();
+    if (!finishes(a)) let_next_start();
     if (!a.tally) return;  // no tallies wanted (a recomputation): no reduction
     if constexpr (sizeof(T) == 4) {
         DF v[4] = {df_of(t_inj), df_of(t_rec), df_of(t_p), df_of(t_n)};
@@ -92,7 +101,7 @@ __global__ void __launch_bounds__(kWideBlock, kWideBlocksPerSm) wide_step_kernel
     WideTally tl;
     wide_sweep(a, a.pos_in, a.neg_in, a.pos_out, a.neg_out, a.dens, a.dens_zero, block * kWideBlock + threadIdx.x,
                blocks * kWideBlock, tl);
-    let_next_start();
+    if (!finishes(a)) let_next_start();
     if (!a.tally) return;
     DF v[4];
     tl.store(v);
@@ -113,21 +122,34 @@ struct StepLink {
 // FP64 units, which an SM shares among its warps: small blocks spread the warps
 // evenly (36^2 x 206: 264 blocks of 256 leave 40 of 152 SMs half the work of the
 // rest). Measured with 90 tracks a step, us a step: 64 threads 19.7, 128 and 256
-// 21.7, 32 23.8; 100^2 x 406 164 either way.
+// 21.7, 32 23.8; 100^2 x 406 164 either way. A step that finishes its own tallies
+// keeps blocks of 256: its last block reads every block's partials (60^2 x 206, lone
+// steps: 49.4 us with 64 threads, 43.5 with 256).
 template <typename T> constexpr int kFlatBlock = sizeof(T) == 8 ? 64 : 256;
+constexpr int kFinishBlock = 256;
 
-// Blocks of a flat step (wide: of the eight-wide form); in a run one block
-// fewer than fit at once, so that the summing block runs beside them.
-static int64_t flat_blocks(const pic_grid *g, bool wide, bool run) {
-    const int64_t items = g->no_xy * g->no_xy * (g->kpitch / (wide ? 8 : 4)), block = wide ? kWideBlock : g->dtype == PIC_F64 ? kFlatBlock<double> : kFlatBlock<float>;
-    const int64_t cap = wide ? (int64_t)kWideBlocksPerSm * sm_count() : step_grid_cap(g->dtype == PIC_F64 ? 1 : 0);
+// Blocks of a flat step (wide: of the eight-wide form; finish: one that
+// finishes its own tallies); in a run one block fewer than fit at once, so that
+// the summing block runs beside them.
+static int64_t flat_blocks(const pic_grid *g, bool wide, bool finish, bool run) {
+    const bool small = g->dtype == PIC_F64 && !finish;
+    const int64_t items = g->no_xy * g->no_xy * (g->kpitch / (wide ? 8 : 4)), block = wide ? kWideBlock : small ? kFlatBlock<double> : kFinishBlock;
+    int64_t cap = wide ? (int64_t)kWideBlocksPerSm * sm_count() : step_grid_cap(g->dtype == PIC_F64 ? 1 : 0);
+    if (g->dtype == PIC_F64 && finish) cap = std::max<int64_t>(1, cap * kFlatBlock<double> / kFinishBlock);
     return std::min({(items + block - 1) / block, std::max<int64_t>(1, cap - (run ? 1 : 0)), kMaxStepBlocks / 2});
+}
+
+template <typename T, int BLOCK>
+static int launch_four_wide(const pic_grid *g, unsigned blocks, const StepArgs<T> &a, cudaStream_t st) {
+    // (items + stride stays below 2^32 on the 32-bit path: items < 2^29)
+    if (flat_index32(g->no_xy, g->kpitch)) launch_linked(step_kernel<T, BLOCK, uint32_t>, blocks, BLOCK, st, a);
+    else launch_linked(step_kernel<T, BLOCK, int64_t>, blocks, BLOCK, st, a);
+    return check_launch("step_kernel");
 }
 
 template <typename T>
 static int launch_step_t(const pic_grid *g, const void *pos_in, const void *neg_in, void *pos_out, void *neg_out,
                          const void *dens, void *dens_zero, double *tally, void *ws, const StepLink *link, cudaStream_t st) {
-    constexpr int BLOCK = kFlatBlock<T>;
     StepArgs<T> a;
     a.pos_in = (const T *)pos_in;
     a.neg_in = (const T *)neg_in;
@@ -160,7 +182,8 @@ static int launch_step_t(const pic_grid *g, const void *pos_in, const void *neg_
     a.div_c4 = make_fastdiv(a.c4);
     a.div_n = make_fastdiv(a.n);
     const bool wide = sizeof(T) == 4 && wide_eligible(g->no_xy, g->kpitch, pos_in, neg_in, pos_out, neg_out);
-    int64_t blocks = flat_blocks(g, wide, link);
+    const bool finish = tally && !(link && link->leave);
+    int64_t blocks = flat_blocks(g, wide, finish, link);
     a.prev_partials = nullptr;
     a.prev_tally = nullptr;
     a.prev_blocks = 0;
@@ -178,12 +201,8 @@ static int launch_step_t(const pic_grid *g, const void *pos_in, const void *neg_
             return check_launch("wide_step_kernel");
         }
     }
-    // (items + stride stays below 2^32 on the 32-bit path: items < 2^29)
-    if (flat_index32(g->no_xy, g->kpitch))
-        launch_linked(step_kernel<T, BLOCK, uint32_t>, (unsigned)blocks, BLOCK, st, a);
-    else
-        launch_linked(step_kernel<T, BLOCK, int64_t>, (unsigned)blocks, BLOCK, st, a);
-    return check_launch("step_kernel");
+    return finish ? launch_four_wide<T, kFinishBlock>(g, (unsigned)blocks, a, st)
+                  : launch_four_wide<T, kFlatBlock<T>>(g, (unsigned)blocks, a, st);
 }
 
 static int launch_flat(const pic_grid *g, const void *pos_in, const void *neg_in, void *pos_out, void *neg_out,
@@ -218,7 +237,7 @@ int StepRun::step(const void *pos_in, const void *neg_in, void *pos_out, void *n
     link.prev_tally = prev_tally_;
     link.prev_blocks = prev_blocks_;
     prev_tally_ = link.leave ? tally : nullptr;
-    prev_blocks_ = (int)flat_blocks(&g_, wide, true);
+    prev_blocks_ = (int)flat_blocks(&g_, wide, !link.leave, true);
     return launch_flat(&g_, pos_in, neg_in, pos_out, neg_out, dens, dens_zero, tally, ws_, &link, st_);
 }
 

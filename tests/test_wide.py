@@ -191,3 +191,38 @@ def test_tall_grids_step_flat(n, no_z, wall, expected):
     g = _grid(native, n, no_z, wall, native.PIC_F32, 0)
     native.check(native.load().pic_segment_resident(ctypes.byref(g), ctypes.byref(out)), "pic_segment_resident")
     assert out.value == expected
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,no_z", [(3, 1), (5, 20), (24, 200), (61, 200)])
+def test_float64_lone_steps_equal_a_segments(n, no_z):
+    """A step that finishes its own tallies (blocks of 256) and a segment's steps
+    (blocks of 64, summed by the next one): the same fields, bit for bit, and the
+    same tallies to the rounding of a sum of 1e6 values of one sign."""
+    import ctypes
+
+    import torch
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    lib = native.load()
+    steps = 3
+    state, xs, ys, off = _case(n, no_z, steps, n, 0)
+    for wall in (0, 1):
+        g = _grid(native, n, no_z, wall, native.PIC_F64, native.PIC_VARIANT_FLAT)
+        whole = _segment(native, g, torch, state, xs, ys, off, 0)
+        f = [torch.zeros((n, n, g.kpitch), dtype=torch.float64, device="cuda") for _ in range(4)]
+        for q in range(2):
+            f[q][:, :, : g.nzb] = torch.from_numpy(state[q])
+        tally = torch.zeros((steps, 4), dtype=torch.float64, device="cuda")
+        b = ctypes.c_int64()
+        native.check(lib.pic_step_workspace_bytes(ctypes.byref(g), ctypes.byref(b)), "pic_step_workspace_bytes")
+        ws = torch.zeros(b.value, dtype=torch.uint8, device="cuda")
+        for s in range(steps):
+            i, o = 2 * (s & 1), 2 * (~s & 1)
+            native.check(lib.pic_step(ctypes.byref(g), f[i].data_ptr(), f[i + 1].data_ptr(), f[o].data_ptr(),
+                                      f[o + 1].data_ptr(), None, None, tally[s].data_ptr(), ws.data_ptr(), ws.numel(),
+                                      torch.cuda.current_stream().cuda_stream), "pic_step")
+        out = 2 * (steps & 1)
+        for q in range(2):
+            assert np.array_equal(f[out + q][:, :, : g.nzb].cpu().numpy(), whole[q])
+        np.testing.assert_allclose(tally.cpu().numpy(), whole[3], rtol=1e6 * 2.0**-53, atol=0)
