@@ -263,3 +263,14 @@ def test_dense_segments_step_flat(n, no_z, tracks, steps, flat):
     for q in range(4):
         assert np.abs(got[3][:, q] - ref[3][:, q]).max() <= tol * np.abs(ref[3][:, q]).max() + 1e-30
     assert np.array_equal(got[4], ref[4])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,tuned", [("column_10um_r008", 0), ("column_5um_r05_d8p91", 1)])
+def test_tuning_leaves_resident_grids_to_the_library(monkeypatch, name, tuned):
+    """The autotuner names a variant, and a grid with one named does not run resident."""
+    autotune = importlib.import_module(pkg().__name__ + ".autotune")
+    calls = []
+    monkeypatch.setattr(autotune, "tune", lambda *a, **kw: calls.append(a))
+    pkg().run_simulation_b200(make_config(name), progress=False, return_fields=False, max_steps=8, tune=True)
+    assert len(calls) == tuned
