@@ -2,8 +2,10 @@
 
 For one grid it times every candidate shape -- the flat kernel, and the
 streaming kernel over tile rows x shared-memory stages x consumer warps x
-resident CTAs per SM x planes per work item -- with CUDA events on the
-launching stream, on the real buffers, and keeps the fastest. Results are
+resident CTAs per SM x planes per work item -- as a segment's steps on the
+launching stream, with CUDA events, on the real buffers, and keeps the fastest.
+Grids that run resident (``engine.runs_resident``) are best left to the library:
+a tuned one names a variant and steps flat; the solver and the gradient ask first. Results are
 cached per (device name, no_xy, nzb, dtype, wall, deposition) in a JSON file so
 a configuration is tuned once per machine.
 
@@ -12,11 +14,11 @@ against shared memory and thread limits); the register file bounds how many
 CTAs of a shape can actually be resident, which the timing then shows.
 
 Steps per launch (temporal blocking in time): when the flat kernel wins, a
-segment of idle steps is also timed as one CUDA graph of per-step launches
-and as cooperative launches of 32 and 256 steps (``steps_per_launch``), and
-the fastest is kept. Measured on GB300 the multi-step launch wins only on
-the smallest grids (24 x 24 x 206: 9.7 against 10.2 us a step) and loses on
-larger ones (48 x 48 x 206: 13.9 against 13.0 us).
+segment of idle steps is also timed as per-step launches and as cooperative
+launches of 32 and 256 steps (``steps_per_launch``), and the fastest is kept.
+Measured on GB300, us a step, per-step / 32 / 256: 10^2 x 56 2.8 / 4.3 / 4.2, 24^2 x
+206 3.3 / 4.3 / 4.2, 48^2 x 206 4.0 / 6.3 / 6.2, 56^2 x 606 7.0 / 10.7 / 10.5, 108^2 x
+206 8.5 / 12.4 / 12.3.
 """
 
 from __future__ import annotations
@@ -89,78 +91,83 @@ def save_cache(d: dict) -> None:
     os.replace(tmp, CACHE)
 
 
+MULTI_CANDIDATES = (32, 256)
+MULTI_TIMED_STEPS = 128
+MULTI_MAX_CELLS = 8_000_000  # larger grids are bandwidth-bound: one launch a step
+SHAPE_STEPS, SHAPE_CELLS = 32, 20_000_000
+
+
 def time_shape(engine, shape: dict, reps: int = 10, warmup: int = 2, with_deposition: bool = True) -> float:
-    """Median milliseconds of one fused step with this launch shape."""
+    """Milliseconds of one step with this launch shape, as segments run it
+    (``pic_run_segment``: steps that overlap their launches and sum their
+    tallies for one another): the faster of two segments of ``reps`` / 2 steps,
+    and on small grids of up to SHAPE_STEPS (SHAPE_CELLS cells in all), so that the device and
+    not the host's first launches are timed. With deposition each step has a
+    track, of no charge, in a histogram of its own: zero fields stay zero."""
     torch = engine.torch
     g = N.PicGrid.from_buffer_copy(engine.grid)
     for k in SHAPE_FIELDS:
         setattr(g, k, 0)
     apply_shape(g, shape)
-    lib = engine.lib
+    g.gaussian_factor = 0.0
+    n = max(1, reps // 2, min(SHAPE_STEPS, SHAPE_CELLS // (int(g.no_xy) ** 2 * int(g.kpitch))))
+    kw = dict(dtype=torch.float64, device=engine.device)
+    xy = torch.full((max(n, warmup),), g.mid_xy, **kw)
+    tally = torch.zeros((max(n, warmup), 4), **kw)
+    dens = [torch.zeros_like(d) for d in engine.dens]
+    counts = torch.zeros_like(engine.counts)
     st = torch.cuda.current_stream(engine.device)
-    dens = engine.dens[0].data_ptr() if with_deposition else None
     cur = engine.parity
+
+    def segment(steps):
+        nonlocal cur
+        off = np.arange(steps + 1, dtype=np.int64) * int(with_deposition)
+        N.check(engine.lib.pic_run_segment(
+            ctypes.byref(g), engine.pos[0].data_ptr(), engine.neg[0].data_ptr(), engine.pos[1].data_ptr(),
+            engine.neg[1].data_ptr(), cur, steps, xy.data_ptr(), xy.data_ptr(), off.ctypes.data, dens[0].data_ptr(),
+            dens[1].data_ptr(), 0, counts.data_ptr(), tally.data_ptr(), engine.workspace.data_ptr(),
+            engine.workspace.numel(), st.cuda_stream), "pic_run_segment")
+        cur ^= steps & 1
+
+    if warmup > 0:
+        segment(warmup)
     times = []
-    for r in range(warmup + reps):
+    for _ in range(2):
         a = torch.cuda.Event(enable_timing=True)
         b = torch.cuda.Event(enable_timing=True)
         a.record(st)
-        rc = lib.pic_step(ctypes.byref(g), engine.pos[cur].data_ptr(), engine.neg[cur].data_ptr(),
-                          engine.pos[cur ^ 1].data_ptr(), engine.neg[cur ^ 1].data_ptr(), dens, None,
-                          engine.tally[0].data_ptr(), engine.workspace.data_ptr(), engine.workspace.numel(),
-                          st.cuda_stream)
-        N.check(rc, "pic_step")
+        segment(n)
         b.record(st)
-        cur ^= 1
-        if r >= warmup:
-            times.append((a, b))
+        times.append((a, b))
     torch.cuda.synchronize(engine.device)
     engine.check_status()
-    return statistics.median(x.elapsed_time(y) for x, y in times)
-
-
-MULTI_CANDIDATES = (32, 256)
-MULTI_TIMED_STEPS = 128
-MULTI_MAX_CELLS = 8_000_000  # larger grids are bandwidth-bound: one launch a step
+    return min(x.elapsed_time(y) for x, y in times) / n
 
 
 def time_segment(engine, steps_per_launch: int, n_steps: int = MULTI_TIMED_STEPS, reps: int = 3) -> float:
     """Median milliseconds per step of ``n_steps`` idle steps with the
-    engine's shape and ``steps_per_launch`` (0: one CUDA graph of per-step
-    launches; K: cooperative launches of up to K steps)."""
+    engine's shape and ``steps_per_launch`` (0: per-step launches; K:
+    cooperative launches of up to K steps)."""
     torch = engine.torch
-    lib = engine.lib
     g = N.PicGrid.from_buffer_copy(engine.grid)
     g.steps_per_launch = int(steps_per_launch)
     st = torch.cuda.current_stream(engine.device)
     off = np.zeros(n_steps + 1, dtype=np.int64)  # no tracks
     tally = torch.zeros((n_steps, 4), dtype=torch.float64, device=engine.device)
-    args = (ctypes.byref(g), engine.pos[0].data_ptr(), engine.neg[0].data_ptr(), engine.pos[1].data_ptr(),
+    times = []
+    for r in range(reps + 1):
+        a = torch.cuda.Event(enable_timing=True)
+        b = torch.cuda.Event(enable_timing=True)
+        a.record(st)
+        N.check(engine.lib.pic_run_segment(
+            ctypes.byref(g), engine.pos[0].data_ptr(), engine.neg[0].data_ptr(), engine.pos[1].data_ptr(),
             engine.neg[1].data_ptr(), 0, n_steps, engine.xs.data_ptr(), engine.ys.data_ptr(), off.ctypes.data,
             engine.dens[0].data_ptr(), engine.dens[1].data_ptr(), 0, engine.counts.data_ptr(), tally.data_ptr(),
-            engine.workspace.data_ptr(), engine.workspace.numel(), st.cuda_stream)
-    graph = None
-    if steps_per_launch <= 1:
-        h = ctypes.c_void_p()
-        N.check(lib.pic_graph_create(*args, ctypes.byref(h)), "pic_graph_create")
-        graph = h.value
-    times = []
-    try:
-        for r in range(reps + 1):
-            a = torch.cuda.Event(enable_timing=True)
-            b = torch.cuda.Event(enable_timing=True)
-            a.record(st)
-            if graph is not None:
-                N.check(lib.pic_graph_launch(graph, st.cuda_stream), "pic_graph_launch")
-            else:
-                N.check(lib.pic_run_segment(*args), "pic_run_segment")
-            b.record(st)
-            if r > 0:
-                times.append((a, b))
-        torch.cuda.synchronize(engine.device)
-    finally:
-        if graph is not None:
-            lib.pic_graph_destroy(graph)
+            engine.workspace.data_ptr(), engine.workspace.numel(), st.cuda_stream), "pic_run_segment")
+        b.record(st)
+        if r > 0:
+            times.append((a, b))
+    torch.cuda.synchronize(engine.device)
     engine.check_status()
     return statistics.median(x.elapsed_time(y) for x, y in times) / n_steps
 

@@ -70,3 +70,61 @@ def test_large_grids_keep_one_launch_a_step(tuner):
     assert "steps_per_launch" not in best["shape"] and calls["segment"] == []
     assert e.grid.steps_per_launch == 0
     assert not (at.CACHE).exists()  # use_cache=False writes nothing
+
+
+def _timing_engine(calls):
+    """An engine without a GPU whose library notes what it is asked to run."""
+    import torch
+
+    class Event:
+        def __init__(self, enable_timing):
+            pass
+
+        def record(self, stream):
+            pass
+
+        def elapsed_time(self, other):
+            return 1.0
+
+    class Library:
+        def __getattr__(self, name):
+            def call(grid, *args):
+                calls.append((name, grid._obj.gaussian_factor, args))
+                return 0
+
+            return call
+
+    cuda = types.SimpleNamespace(Event=Event, current_stream=lambda dev: types.SimpleNamespace(cuda_stream=0),
+                                 synchronize=lambda dev: None)
+    e = _engine("column_10um_r008")
+    field = lambda: torch.zeros(8)  # noqa: E731
+    e.torch = types.SimpleNamespace(cuda=cuda, zeros=torch.zeros, full=torch.full, zeros_like=torch.zeros_like,
+                                    float64=torch.float64)
+    e.device, e.lib, e.parity = "cpu", Library(), 0
+    e.pos, e.neg, e.dens = ([field(), field()] for _ in range(3))
+    e.xs, e.ys, e.counts, e.workspace = field(), field(), field(), field()
+    e.check_status = lambda: None
+    return e
+
+
+@pytest.mark.parametrize("with_deposition", [True, False])
+def test_shapes_are_timed_as_segments_run_them(with_deposition):
+    """Steps of a segment overlap their launches and sum their tallies for one
+    another; a lone step does neither. The tracks timed with add no charge and
+    touch neither the engine's histogram nor its pairs."""
+    at = importlib.import_module(pkg().__name__ + ".autotune")
+    calls = []
+    e = _timing_engine(calls)
+    assert at.time_shape(e, {"variant": "flat"}, reps=10, with_deposition=with_deposition) == 1.0 / 32
+    assert [name for name, _, _ in calls] == ["pic_run_segment"] * 3
+    assert [args[5] for _, _, args in calls] == [2, 32, 32]  # steps: warm-up, two timed segments of a small grid
+    for _, gfac, args in calls:
+        assert gfac == 0.0
+        assert e.counts.data_ptr() not in args and not {d.data_ptr() for d in e.dens} & set(args)
+
+
+def test_per_step_launches_are_timed_as_runs_issue_them():
+    at = importlib.import_module(pkg().__name__ + ".autotune")
+    calls = []
+    at.time_segment(_timing_engine(calls), 0, n_steps=16, reps=2)
+    assert [name for name, _, _ in calls] == ["pic_run_segment"] * 3  # no graph is replayed by default
