@@ -6,8 +6,8 @@ resident CTAs per SM x planes per work item -- as a segment's steps on the
 launching stream, with CUDA events, on the real buffers, and keeps the fastest.
 Grids that run resident (``engine.runs_resident``) are best left to the library:
 a tuned one names a variant and steps flat; the solver and the gradient ask first. Results are
-cached per (device name, no_xy, nzb, dtype, wall, deposition) in a JSON file so
-a configuration is tuned once per machine.
+cached per (device name, kernel sources, no_xy, nzb, dtype, wall, deposition) in
+a JSON file so a configuration is tuned once per machine and library.
 
 Only shapes the library accepts are timed (``pic_resolve_shape`` checks them
 against shared memory and thread limits); the register file bounds how many
@@ -24,6 +24,8 @@ Measured on GB300, us a step, per-step / 32 / 256: 10^2 x 56 2.8 / 4.3 / 4.2, 24
 from __future__ import annotations
 
 import ctypes
+import functools
+import hashlib
 import itertools
 import json
 import os
@@ -33,6 +35,7 @@ from pathlib import Path
 import numpy as np
 
 from . import _native as N
+from . import build as _build
 from .engine import SHAPE_FIELDS, apply_shape, resolve_shape
 
 CACHE = Path(os.environ.get("PIC_TUNE_CACHE", Path(__file__).resolve().parent / "_build" / "tuning.json"))
@@ -70,11 +73,20 @@ def candidate_shapes(grid, quick: bool = False) -> list[dict]:
     return out
 
 
+@functools.lru_cache(maxsize=1)
+def _kernels() -> str:
+    """What the library is built from: a shape measured on other kernels is not reused."""
+    h = hashlib.sha256()
+    for p in sorted([*_build.CSRC.glob("*.cu"), *_build.CSRC.glob("*.cuh"), *_build.CSRC.glob("*.h")]):
+        h.update(p.name.encode() + b"\0" + p.read_bytes() + b"\0")
+    return h.hexdigest()[:16]
+
+
 def _key(grid, with_deposition: bool) -> str:
     import torch
 
     name = torch.cuda.get_device_name()
-    return f"{name}|{grid.no_xy}|{grid.nzb}|{grid.dtype}|{grid.wall}|{int(with_deposition)}"
+    return f"{name}|{_kernels()}|{grid.no_xy}|{grid.nzb}|{grid.dtype}|{grid.wall}|{int(with_deposition)}"
 
 
 def load_cache() -> dict:

@@ -128,3 +128,16 @@ def test_per_step_launches_are_timed_as_runs_issue_them():
     calls = []
     at.time_segment(_timing_engine(calls), 0, n_steps=16, reps=2)
     assert [name for name, _, _ in calls] == ["pic_run_segment"] * 3  # no graph is replayed by default
+
+
+def test_shapes_measured_on_other_kernels_are_not_reused(tuner, monkeypatch):
+    import torch
+
+    at, calls, _ = tuner
+    monkeypatch.undo()  # the real key
+    monkeypatch.setattr(torch.cuda, "get_device_name", lambda: "test")
+    g = _engine("column_10um_r008").grid
+    key = at._key(g, True)
+    assert key == at._key(g, True) and key != at._key(g, False)
+    monkeypatch.setattr(at, "_kernels", lambda: "other sources")
+    assert at._key(g, True) != key
