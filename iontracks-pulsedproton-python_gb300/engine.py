@@ -101,7 +101,8 @@ def make_grid(config, dtype: str = "float32", alpha_cm3_s: float | None = None, 
 
 
 def device_bytes(config, dtype: str = "float32", max_tracks: int = 0) -> int:
-    """HBM the engine allocates for a configuration."""
+    """HBM the engine allocates for a configuration's fields, pairs, histogram,
+    tallies and tracks (its workspace, 35 to 220 MB, comes on top)."""
     n = int(config.no_xy)
     kp = (int(config.no_z_with_buffer) + 7) // 8 * 8
     es = 4 if dtype == "float32" else 8
@@ -153,6 +154,20 @@ class ChamberEngine:
         self.parity = 0  # fields[parity] holds the current state
         self.step_index = 0  # global step of the next call
         self._graphs = {}
+
+    def use_step_workspace(self) -> None:
+        """Gives back what ``pic_segment_workspace_bytes`` adds to the step
+        workspace (20 to 200 MB on small grids): segments then run one launch a
+        step."""
+        b = ctypes.c_int64()
+        N.check(self.lib.pic_step_workspace_bytes(ctypes.byref(self.grid), ctypes.byref(b)), "pic_step_workspace_bytes")
+        if self.workspace.numel() <= int(b.value):
+            return
+        self.check_status()  # (synchronises: nothing uses the old one any more)
+        self.close()  # graphs hold its address
+        self.workspace = None
+        self.torch.cuda.empty_cache()
+        self.workspace = self.torch.zeros(int(b.value), dtype=self.torch.uint8, device=self.device)
 
     # ---- tracks --------------------------------------------------------
     def ensure_track_capacity(self, n: int) -> None:

@@ -274,3 +274,33 @@ def test_tuning_leaves_resident_grids_to_the_library(monkeypatch, name, tuned):
     monkeypatch.setattr(autotune, "tune", lambda *a, **kw: calls.append(a))
     pkg().run_simulation_b200(make_config(name), progress=False, return_fields=False, max_steps=8, tune=True)
     assert len(calls) == tuned
+
+
+@pytest.mark.gpu
+def test_gradient_within_the_memory_a_step_workspace_leaves():
+    """A memory_limit that holds the fields, the step workspace, lambda and the
+    segment schedule is enough: the resident steps' workspace is given back then."""
+    import torch
+
+    adj = importlib.import_module(pkg().__name__ + ".adjoint")
+    native = importlib.import_module(pkg().__name__ + "._native")
+    cfg = make_config("column_10um_r008")
+    free = adj.AdjointRun(cfg, max_steps=200)
+    ks = free.forward()
+    grad = free.backward()
+    eng, step = free._eng, ctypes.c_int64()
+    native.check(native.load().pic_step_workspace_bytes(ctypes.byref(eng.grid), ctypes.byref(step)), "bytes")
+    assert eng.workspace.numel() > step.value
+    rest = (*eng.pos, *eng.neg, *eng.dens, eng.counts, eng.tally, eng.xs, eng.ys)
+    held = sum(t.numel() * t.element_size() for t in rest) + step.value
+    own = sum(t.numel() * t.element_size() for t in (free.ckpt, free.dens_keep))
+    states = 2 * (free.K + 2) * free.field * 4  # the segment's states and lambda
+    free.release()
+    for schedule in ("segments", "auto"):
+        run = adj.AdjointRun(cfg, max_steps=200, memory_limit=held + own + states, schedule=schedule)
+        assert abs(run.forward() - ks) <= 1e-6 * ks and run.kind == "segments"
+        np.testing.assert_allclose(run.backward(), grad, rtol=1e-4)
+        run.release()
+    with pytest.raises(MemoryError):
+        adj.AdjointRun(cfg, max_steps=200, memory_limit=held + own + states - 4, schedule="segments").forward()
+    torch.cuda.synchronize()
