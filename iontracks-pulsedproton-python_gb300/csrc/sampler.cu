@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <memory>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -162,11 +163,13 @@ void arrival_counts_serial(Pcg64 start, int64_t n, double duration, const double
 // 5 000 0.07 / 0.11: worth it from about 32 draws a bin.
 constexpr int kArrivalBlock = 32;
 
-void arrival_counts_blocks(Pcg64 start, int64_t n, double duration, const double *edges, int64_t n_edges,
+// False: no memory for the blocks (nothing drawn).
+bool arrival_counts_blocks(Pcg64 start, int64_t n, double duration, const double *edges, int64_t n_edges,
                            int64_t *counts, Pcg64 &end) {
     const int64_t blocks = (n + kArrivalBlock - 1) / kArrivalBlock, nb = n_edges - 1;
-    std::vector<double> before((size_t)blocks + 1);
-    std::vector<u128> state((size_t)blocks);
+    const std::unique_ptr<double[]> before(new (std::nothrow) double[(size_t)blocks + 1]);
+    const std::unique_ptr<u128[]> state(new (std::nothrow) u128[(size_t)blocks]);
+    if (!before || !state) return false;
     const u128 m2 = kPcgMult * kPcgMult, c2 = (kPcgMult + 1) * start.inc, m4 = m2 * m2, c4 = (m2 + 1) * c2;
     auto output = [](u128 s) {
         const uint64_t x = (uint64_t)(s >> 64) ^ (uint64_t)s;
@@ -245,6 +248,7 @@ void arrival_counts_blocks(Pcg64 start, int64_t n, double duration, const double
     }
     end.state = s;
     end.inc = start.inc;
+    return true;
 }
 
 }  // namespace
@@ -257,8 +261,8 @@ int arrival_counts_pcg64(uint64_t *st, int64_t n, double duration, const double 
     const unsigned hw = std::thread::hardware_concurrency();
     const int64_t threads = std::min<int64_t>(std::max<unsigned>(hw, 1u), 64);
     if (n < kArrivalThreadedMin || threads < 2) {
-        if (n >= 32 * n_edges) arrival_counts_blocks(start, n, duration, edges, n_edges, counts, end);
-        else arrival_counts_serial(start, n, duration, edges, n_edges, counts, end);
+        if (n < 32 * n_edges || !arrival_counts_blocks(start, n, duration, edges, n_edges, counts, end))
+            arrival_counts_serial(start, n, duration, edges, n_edges, counts, end);
     } else {
         std::unique_ptr<double[]> S(new double[(size_t)n]);
         double *u = S.get();

@@ -196,3 +196,38 @@ def test_schedules_drawn_on_threads_equal_the_sequential_ones():
     for a, b, ra, rb in zip(seq, par, seq_rngs, par_rngs):
         np.testing.assert_array_equal(a, b)
         assert ra.bit_generator.state == rb.bit_generator.state
+
+
+_ARRIVALS_WITHOUT_MEMORY = """
+import ctypes, resource, sys
+lib = ctypes.CDLL(sys.argv[1])
+n, bins = 1_000_000, 100
+lib.pic_arrival_counts_pcg64.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_double, ctypes.c_void_p,
+                                         ctypes.c_int64, ctypes.c_void_p]
+edges = (ctypes.c_double * (bins + 1))(*[5.4e-4 * b / bins for b in range(bins + 1)])
+states = [(ctypes.c_uint64 * 4)(1, 2, 3, 5) for _ in range(2)]
+counts = [(ctypes.c_int64 * bins)() for _ in range(2)]
+call = lambda k: lib.pic_arrival_counts_pcg64(states[k], n, 5.4e-4, edges, bins + 1, counts[k])
+rcs = [call(0), 0]
+libc = ctypes.CDLL(None)
+libc.malloc.restype, libc.malloc.argtypes = ctypes.c_void_p, [ctypes.c_size_t]
+vm = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (vm, vm))
+for size in (1 << 20, 1 << 18, 1 << 17, 1 << 16):
+    while libc.malloc(size):
+        pass
+rcs[1] = call(1)
+sys.exit(0 if rcs == [0, 0] and list(counts[0]) == list(counts[1]) and list(states[0]) == list(states[1]) else 3)
+"""
+
+
+def test_arrivals_are_counted_without_memory_for_blocks():
+    """No C++ exception leaves the C entry: without memory for the blocks' sums the
+    draws are made twice instead, with the same counts and generator state."""
+    import subprocess
+    import sys
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    native.load()
+    done = subprocess.run([sys.executable, "-c", _ARRIVALS_WITHOUT_MEMORY, str(native.library_path())], capture_output=True)
+    assert done.returncode == 0, done
