@@ -1,7 +1,7 @@
 // resident.cu -- up to kResSteps time steps of a small float32 grid in ONE
 // cooperative launch whose blocks keep the fields on the chip.
 //
-// A grid of up to a few million cells has less state than the SMs have
+// A grid of up to about 1.7 million cells has less state than the SMs have
 // registers and shared memory, but launched step by step it is rewritten
 // through L2 every step, and a step costs two chains of L2 round trips (its
 // neighbour loads, its tally reduction) and a launch gap: 5-15 us whatever
@@ -36,8 +36,8 @@
 // through L2, the rest the patches' arithmetic and shared memory at 65 cycles a
 // warp's item -- not bandwidth. Measured on GB300, us a step of a 256-step
 // launch without tracks, against the flat step's launches: 11^2 x 56 1.6 (6.2),
-// 24^2 x 206 2.1 (8.3), 48^2 x 206 2.8 (8.3), 53^2 x 206 3.0 (10.3), 76^2 x 206
-// 5.0 (12.4), 48^2 x 406 3.6 (10.3), 59^2 x 406 5.5 (12.4); with 14 tracks a step
+// 24^2 x 206 2.1 (8.3), 48^2 x 206 2.8 (8.3), 53^2 x 206 3.1 (10.3), 76^2 x 206
+// 5.0 (12.4), 48^2 x 406 3.6 (10.3), 59^2 x 406 5.4 (12.4); with 14 tracks a step
 // on 24^2 x 206, their deposition included, 2.4.
 //
 // The arithmetic is the streaming step's (pic_stream.cuh; the reference's
@@ -74,12 +74,22 @@ __device__ __forceinline__ DF two_sum(float a, float b) {
     return DF{s, (a - (s - v)) + (b - v)};
 }
 
+// Adds an item's sum (a scored one's) to a thread's tally of a step, the first as it is.
+__device__ __forceinline__ void tally_item(Tally<float> &t, float2 v, bool scored, bool first) {
+    const float x = scored ? v.x + v.y : 0.f;
+    if (first) t.s = x;
+    else t.add(x);
+}
+
 // Shared memory: two buffers of deposition pairs over the block's columns (ring
-// and halo included), two buffers of the threads' tallies, one or two buffers
-// of the cells ([row][column][species][4 + 4 TKV] and 4 floats more, a row and a
+// and halo included), the threads' tallies (of a patch of several items
+// double-floats; two buffers where no barrier stands between the sum of a step's,
+// at the next one's start, and that one's own), one or two buffers of the cells ([row][column][species][4 + 4 TKV] and 4 floats more, a row and a
 // column more on each side), and the table of what the block trades.
 __host__ __device__ inline int res_pair_floats(int cells) { return (4 * cells + 3) / 4 * 4; }
 __host__ __device__ constexpr bool res_small(int ri, int rj) { return ri * rj < 6; }
+__host__ __device__ constexpr int res_tally_values(int ri, int rj) { return ri * rj > 1 ? 2 : 1; }
+__host__ __device__ inline int res_tally_buffers(bool small, int blocks) { return small && blocks == 1 ? 2 : 1; }
 template <int RI, int RJ, int TKV, int MAXT, bool MIRROR>
 __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant__ ResArgs a) {
     // Small patches keep two buffers of cells, so that a step's values need not
@@ -98,15 +108,17 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
     const int n = a.n, kp = a.kp, tkv = a.tkv, steps = a.steps;
     const int ncell = res_cells(a.gi, a.gj, RI, RJ);
     float2 *pairs = reinterpret_cast<float2 *>(res_smem);  // [2][ncell]
-    float *sums = res_smem + res_pair_floats(ncell);       // [2][3][T]
-    float *S = sums + 6 * T;
+    constexpr int VALUES = res_tally_values(RI, RJ);
+    float *const sums = res_smem + res_pair_floats(ncell);  // [1 or 2][3][T][VALUES]
+    const int SUMS = res_tally_buffers(SMALL, gridDim.x) == 2 ? 3 * VALUES * T : 0;  // from one buffer to the other
+    float *S = sums + 3 * VALUES * T + SUMS;
     const int BUF = SMALL ? ncell * COL + 4 : 0;  // floats from one buffer of cells to the other
     const bool trades = gridDim.x > 1;  // cells with other blocks
 
     // ---- load: cells to zero, then the block's values and its surroundings ----
     if (tid == 0) s_abort = 0;
     for (int u = tid; u < (ncell * COL + 4) / 4 * (SMALL ? 2 : 1); u += blockDim.x) st4s(S + 4 * u, make_float4(0.f, 0.f, 0.f, 0.f));
-    for (int u = tid; u < 6 * T; u += blockDim.x) sums[u] = 0.f;
+    for (int u = tid; u < 3 * VALUES * T + SUMS; u += blockDim.x) sums[u] = 0.f;
     __syncthreads();
     for (int u = tid; u < n_around * kvn; u += blockDim.x) {
         const int col = u / kvn, v = u - col * kvn;
@@ -144,13 +156,14 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
         };
         DF inj{0.f, 0.f};
         auto sum_step = [&](int s) {  // this warp's share of the block's tallies of step s
-            const float *q = sums + (s & 1) * 3 * T;
+            const float *q = sums + (s & 1) * SUMS;
             DF v[4] = {inj, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
-            for (int u = 4 * at; u < T; u += 4 * AT)
+            for (int u = 4 / VALUES * at; u < T; u += 4 / VALUES * AT)
 #pragma unroll
                 for (int x = 0; x < 3; ++x) {
-                    const float4 f = ld4s(q + x * T + u);
-                    v[x + 1] = df_add(v[x + 1], df_add(two_sum(f.x, f.y), two_sum(f.z, f.w)));
+                    const float4 f = ld4s(q + VALUES * (x * T + u));
+                    v[x + 1] = df_add(v[x + 1], VALUES == 1 ? df_add(two_sum(f.x, f.y), two_sum(f.z, f.w))
+                                                            : df_add(DF{f.x, f.y}, DF{f.z, f.w}));
                 }
             const DF w = warp_sum4(v, lane);
             if ((lane & 7) == 0)
@@ -272,7 +285,7 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
     // store in it: the items' loads and arithmetic overlap.
     auto advance = [&](auto with_deposition, const float *cells, const float2 *Dp) {
         constexpr bool DEP = decltype(with_deposition)::value;
-        float2 t_rec = make_float2(0.f, 0.f);
+        Tally<float> t_rec;
         float4 pP[RJ], pN[RJ];  // the row before, as it was (large patches: from the cells, which still hold it)
         if (SMALL)
 #pragma unroll
@@ -335,7 +348,7 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
                 P[r][c] = make_float4(plo.x, plo.y, phi.x, phi.y);
                 N[r][c] = make_float4(nlo.x, nlo.y, nhi.x, nhi.y);
                 const float2 rec = gap_sum(make_float4(rlo.x, rlo.y, rhi.x, rhi.y));
-                if (scored >> (r * RJ + c) & 1) t_rec = __fadd2_rn(t_rec, rec);
+                tally_item(t_rec, rec, scored >> (r * RJ + c) & 1, r + c == 0);
             }
             if (SMALL)
 #pragma unroll
@@ -357,7 +370,7 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
         now = BUF - now;
         float *const next = cell0 + now;
         const bool send = s + 1 < steps;
-        const float2 t_rec = a.slot[s] >= 0 ? advance(std::true_type{}, cells, pair0 + pair_now)
+        const Tally<float> t_rec = a.slot[s] >= 0 ? advance(std::true_type{}, cells, pair0 + pair_now)
                                             : advance(std::false_type{}, cells, pair0);
         if (!all_valid) {  // the end planes and the row padding stay zero
             const int top = a.nzb - 2 - k0;  // the last valid element
@@ -405,17 +418,22 @@ __global__ void __launch_bounds__(MAXT, 1) resident_kernel(const __grid_constant
         }
         // while the packets are on their way: the tallies (the aux warps sum
         // them during the next step), the wall's ring, the states to keep
-        float2 t_p = make_float2(0.f, 0.f), t_n = make_float2(0.f, 0.f);
+        Tally<float> t_p, t_n;
 #pragma unroll
         for (int r = 0; r < RI; ++r)
 #pragma unroll
             for (int c = 0; c < RJ; ++c) {
-                const float2 p2 = gap_sum(P[r][c]), n2 = gap_sum(N[r][c]);
-                if (scored >> (r * RJ + c) & 1) t_p = __fadd2_rn(t_p, p2), t_n = __fadd2_rn(t_n, n2);
+                const bool in = scored >> (r * RJ + c) & 1;
+                tally_item(t_p, gap_sum(P[r][c]), in, r + c == 0);
+                tally_item(t_n, gap_sum(N[r][c]), in, r + c == 0);
             }
-        float *const m = sums + sum_now + tid;
-        m[0] = t_rec.x + t_rec.y, m[T] = t_p.x + t_p.y, m[2 * T] = t_n.x + t_n.y;
-        sum_now = 3 * T - sum_now;
+        auto leave = [&](int x, const Tally<float> &t) {
+            float *const m = sums + sum_now + VALUES * (x * T + tid);
+            if constexpr (VALUES == 1) *m = t.s;
+            else *reinterpret_cast<float2 *>(m) = make_float2(t.s, -t.c);
+        };
+        leave(0, t_rec), leave(1, t_p), leave(2, t_n);
+        sum_now = SUMS - sum_now;
         if (a.keep_stride > 0 || !send) {
 #pragma unroll
             for (int r = 0; r < RI; ++r)
@@ -461,7 +479,8 @@ constexpr ResPatch kPatches[] = {{1, 1, 640}, {2, 1, 512}, {2, 2, 512}, {3, 2, 4
 
 int64_t step_smem(const ResPlan &p, const ResPatch &pt) {
     const int64_t cells = res_cells(p.gi, p.gj, pt.ri, pt.rj);
-    return 4 * (res_pair_floats((int)cells) + 6LL * p.threads +
+    const int64_t tallies = 3LL * res_tally_values(pt.ri, pt.rj) * res_tally_buffers(res_small(pt.ri, pt.rj), p.blocks);
+    return 4 * (res_pair_floats((int)cells) + tallies * p.threads +
                 (2 * cells * res_pitch(kResTkvMax) + 4) * (res_small(pt.ri, pt.rj) ? 2 : 1)) +
            16LL * (2 * (p.ti + p.tj) * p.tkv + 2 * p.ti * p.tj);
 }

@@ -304,3 +304,28 @@ def test_gradient_within_the_memory_a_step_workspace_leaves():
     with pytest.raises(MemoryError):
         adj.AdjointRun(cfg, max_steps=200, memory_limit=held + own + states - 4, schedule="segments").forward()
     torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("n,no_z", [(5, 20), (24, 200), (48, 200), (53, 200), (59, 400), (76, 200)])
+def test_tallies_lose_no_bits(n, no_z, variant):
+    """Beyond the four k of an item the tallies are summed in double-floats: of
+    integers below 2^22, of which four add up exactly in float32, they are exact.
+    A step of weight one keeps P = 2 m and halves it where it meets N = 1/2."""
+    import torch
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    g = _grid(native, n, no_z, 0, native.PIC_F32, variant)
+    g.p_lat = g.p_zm = g.p_zp = g.n_lat = g.n_zm = g.n_zp = 0.0
+    g.p_cen = g.n_cen = g.alpha_dt = 1.0
+    m = np.random.default_rng(n).integers(0, 1 << 21, (n, n, no_z + 4)).astype(np.float64)
+    m[:, :, 0] = m[:, :, -1] = 0
+    half = np.zeros_like(m)
+    half[:, :, 1:-1] = 0.5
+    tally = _segment(native, g, torch, [2 * m, half], np.zeros(1), np.zeros(1), np.zeros(5, dtype=np.int64), 0)[3][0]
+    i = np.arange(1, n - 1)
+    scored = (i[:, None] - g.mid_xy) ** 2 + (i[None, :] - g.mid_xy) ** 2 < g.scoring_radius_sq
+    inside = m[1:-1, 1:-1, g.nze : g.nze + no_z][scored]
+    assert inside.size and inside.sum() < 2**44
+    assert np.array_equal(tally, [0.0, inside.sum(), inside.sum(), (0.5 - inside).sum()])
