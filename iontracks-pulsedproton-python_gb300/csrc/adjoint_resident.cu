@@ -255,7 +255,6 @@ __global__ void __launch_bounds__(MAXT, 1) adjoint_resident_kernel(const __grid_
     // lambda_s, with the reflecting ring's share folded in where `fold`.
     auto retreat = [&](auto with_deposition, const float *cells, const float2 *Dp, const float *ringu, bool fold) {
         constexpr bool DEP = decltype(with_deposition)::value;
-        float2 G0 = make_float2(0.f, 0.f), G1 = G0, G2 = G0, G3 = G0, G4 = G0;
         float4 pP[RJ], pN[RJ];
 #pragma unroll
         for (int c = 0; c < RJ; ++c) {
@@ -273,6 +272,7 @@ __global__ void __launch_bounds__(MAXT, 1) adjoint_resident_kernel(const __grid_
 #pragma unroll
             for (int c = 0; c < RJ; ++c) {
                 const float *const d = cells + r * ROW + c * COL;
+                float2 G0 = make_float2(0.f, 0.f), G1 = G0, G2 = G0, G3 = G0, G4 = G0;  // the item's terms
                 const float4 MP = oP[c], MN = oN[c];
                 const float mp_km = d[-1], mp_kp = d[4], mn_km = d[PITCH - 1], mn_kp = d[PITCH + 4];
                 float4 A1, B1, A2, B2, A3, B3;
@@ -353,6 +353,11 @@ __global__ void __launch_bounds__(MAXT, 1) adjoint_resident_kernel(const __grid_
                 }
                 P[r][c] = make_float4(lpl.x, lpl.y, lph.x, lph.y);
                 N[r][c] = make_float4(lnl.x, lnl.y, lnh.x, lnh.y);
+                acc[0].add(G0.x + G0.y);
+                acc[1].add(G1.x + G1.y);
+                acc[2].add(G2.x + G2.y);
+                acc[3].add(G3.x + G3.y);
+                acc[4].add(G4.x + G4.y);
             }
 #pragma unroll
             for (int c = 0; c < RJ; ++c) {
@@ -360,11 +365,6 @@ __global__ void __launch_bounds__(MAXT, 1) adjoint_resident_kernel(const __grid_
                 pN[c] = oN[c];
             }
         }
-        acc[0].add(G0.x + G0.y);
-        acc[1].add(G1.x + G1.y);
-        acc[2].add(G2.x + G2.y);
-        acc[3].add(G3.x + G3.y);
-        acc[4].add(G4.x + G4.y);
     };
 
     int now = 0, pair_now = 0, ring_now = 0;

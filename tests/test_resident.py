@@ -329,3 +329,48 @@ def test_tallies_lose_no_bits(n, no_z, variant):
     inside = m[1:-1, 1:-1, g.nze : g.nze + no_z][scored]
     assert inside.size and inside.sum() < 2**44
     assert np.array_equal(tally, [0.0, inside.sum(), inside.sum(), (0.5 - inside).sum()])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("n,no_z", [(5, 20), (24, 200), (31, 100), (48, 200), (53, 200)])
+def test_derivative_sums_lose_no_bits(n, no_z, variant):
+    """The same of the reverse sweep: with weights of one and no recombination
+    lambda stays what it is, and dR/da adds (1 - lambda+ - lambda-) p n over p = n =
+    1: integers of which four add up exactly in float32, the rest in double-floats."""
+    import torch
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    lib = native.load()
+    steps = every = 8
+    kp = (no_z + 4 + 7) // 8 * 8
+    g = _grid(native, n, no_z, 0, native.PIC_F32, 0)
+    g.adjoint_variant = variant
+    g.p_lat = g.p_zm = g.p_zp = g.n_lat = g.n_zm = g.n_zp = g.alpha_dt = 0.0
+    g.p_cen = g.n_cen = 1.0
+    lam = np.zeros((2, 2, n, n, kp))
+    lam[0, :, 1:-1, 1:-1, 1 : no_z + 3] = np.random.default_rng(n).integers(0, 1 << 21, (2, n - 2, n - 2, no_z + 2))
+    one = np.zeros((2, 1, n, n, kp))
+    one[..., 1 : no_z + 3] = 1.0
+    dev = lambda a: torch.from_numpy(a).to("cuda", torch.float32)  # noqa: E731
+    ckpt, L = dev(one), dev(lam)
+    states = torch.zeros((2, every, n, n, kp), device="cuda")
+    grad = torch.zeros(5, dtype=torch.float64, device="cuda")
+    ws = []
+    for name in ("pic_segment_workspace_bytes", "pic_adjoint_workspace_bytes"):
+        b = ctypes.c_int64()
+        native.check(getattr(lib, name)(ctypes.byref(g), ctypes.byref(b)), name)
+        ws.append(torch.zeros(b.value, dtype=torch.uint8, device="cuda"))
+    off = np.zeros(steps + 1, dtype=np.int64)
+    before = lib.pic_kernel_launches()
+    native.check(lib.pic_adjoint_backward(
+        ctypes.byref(g), ckpt[0].data_ptr(), ckpt[1].data_ptr(), n * n * kp, steps, every, off.ctypes.data, None,
+        states[0].data_ptr(), states[1].data_ptr(), L[0, 0].data_ptr(), L[0, 1].data_ptr(), L[1, 0].data_ptr(),
+        L[1, 1].data_ptr(), grad.data_ptr(), ws[0].data_ptr(), ws[0].numel(), ws[1].data_ptr(), ws[1].numel(),
+        torch.cuda.current_stream().cuda_stream), "pic_adjoint_backward")
+    assert lib.pic_kernel_launches() - before == (steps if variant else 1) + 2  # and the states, the final sum
+    i = np.arange(1, n - 1)
+    scored = (i[:, None] - g.mid_xy) ** 2 + (i[None, :] - g.mid_xy) ** 2 < g.scoring_radius_sq
+    want = steps * (scored.sum() * no_z - lam[0].sum())
+    assert abs(want) < 2**44 and grad[4].item() == want
+    assert np.array_equal(L[steps & 1].cpu().numpy(), lam[0])
