@@ -105,11 +105,14 @@ int resolve_shape(pic_grid *g) {
     // against streaming in its 13-consumer-warp form): 330^2 x 406 123 / - vs
     // 156 / -, 536^2 x 406 317 / 325 vs 347 / 352, 680^2 x 406 (189 M cells) 515 / 525
     // vs 527 / 535, 740^2 x 406 (223 M) 607 / 617 vs 605 / 611, 1068^2 x 406 1320 vs
-    // 1195.
-    if (g->variant == PIC_VARIANT_AUTO)
-        g->variant = (g->dtype == PIC_F32 && g->no_xy >= 64 && g->no_xy * g->no_xy * g->kpitch >= kStreamMinCells)
-                         ? PIC_VARIANT_STREAM
-                         : PIC_VARIANT_FLAT;
+    // 1195. Launch-shape fields are the streaming step's: a caller who sets one
+    // gets that step, and its checks, from half as many cells on.
+    if (g->variant == PIC_VARIANT_AUTO) {
+        const bool shaped = g->tile_rows > 0 || g->planes_per_item > 0 || g->stages > 0 || g->consumer_warps > 0 || g->ctas_per_sm > 0;
+        const int64_t from = shaped ? kStreamMinCells / 2 : kStreamMinCells;
+        g->variant = (g->dtype == PIC_F32 && g->no_xy >= 64 && g->no_xy * g->no_xy * g->kpitch >= from) ? PIC_VARIANT_STREAM
+                                                                                                       : PIC_VARIANT_FLAT;
+    }
     if (g->variant == PIC_VARIANT_FLAT) return PIC_OK;
     if (g->variant != PIC_VARIANT_STREAM) return set_error(PIC_E_INVALID, "variant must be PIC_VARIANT_AUTO, _FLAT or _STREAM");
     if (g->dtype != PIC_F32) return set_error(PIC_E_INVALID, "the stream variant supports float32 fields only");

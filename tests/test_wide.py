@@ -226,3 +226,22 @@ def test_float64_lone_steps_equal_a_segments(n, no_z):
         for q in range(2):
             assert np.array_equal(f[out + q][:, :, : g.nzb].cpu().numpy(), whole[q])
         np.testing.assert_allclose(tally.cpu().numpy(), whole[3], rtol=1e6 * 2.0**-53, atol=0)
+
+
+@pytest.mark.parametrize("n,shape,variant", [(608, {}, 1), (608, dict(tile_rows=8), 2), (608, dict(ctas_per_sm=1), 2),
+                                             (330, dict(tile_rows=8), 1), (1068, {}, 2)])
+def test_a_shape_asks_for_the_streaming_step(n, shape, variant):
+    """AUTO of 1e8 to 2e8 cells steps flat, but not where the caller gives the
+    streaming step a shape, which is checked as ever."""
+    import ctypes
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    g = _grid(native, n, 400, 0, native.PIC_F32, 0)
+    for k, v in shape.items():
+        setattr(g, k, v)
+    out = native.PicGrid()
+    native.check(native.load().pic_resolve_shape(ctypes.byref(g), ctypes.byref(out)), "pic_resolve_shape")
+    assert out.variant == variant
+    g.consumer_warps = 99
+    refused = native.load().pic_resolve_shape(ctypes.byref(g), ctypes.byref(out)) != native.PIC_OK
+    assert refused == (n * n * g.kpitch >= 10**8)
