@@ -409,6 +409,18 @@ int pic_revolve_backward(const pic_grid *g, void *slots_pos, void *slots_neg, in
 int pic_selftest_waits(int32_t *barrier_status, int32_t *mbarrier_status, uintptr_t stream);
 
 /*
+ * pic_selftest_packets -- the same for the third bounded wait: the resident
+ * step and, where lambda fits the chip too, its adjoint, over zero fields of the
+ * grid's size without the last of the division's blocks, whose packets never
+ * come. Returns the status codes they leave after about a second (7; -1 for an
+ * adjoint that does not fit) and whether every block of the adjoint left NaN in
+ * its derivative sums. Refused for a grid that does not run resident in at least
+ * 3 blocks.
+ */
+int pic_selftest_packets(const pic_grid *g, int32_t *step_status, int32_t *adjoint_status, int32_t *poisoned,
+                         uintptr_t stream);
+
+/*
  * pic_capture_begin / pic_capture_end -- record every launch the library
  * issues on `stream` between the two calls (made from this host thread) into
  * a CUDA graph, instantiated and returned in *graph_out (replay with

@@ -791,6 +791,14 @@ int pic_selftest_waits(int32_t *barrier_status, int32_t *mbarrier_status, uintpt
     return selftest_waits(barrier_status, mbarrier_status, reinterpret_cast<cudaStream_t>(stream));
 }
 
+int pic_selftest_packets(const pic_grid *g, int32_t *step_status, int32_t *adjoint_status, int32_t *poisoned,
+                         uintptr_t stream) {
+    int rc = check_grid(g);
+    if (rc) return rc;
+    if (!step_status || !adjoint_status || !poisoned) return set_error(PIC_E_INVALID, "null pointer argument");
+    return selftest_packets(g, step_status, adjoint_status, poisoned, reinterpret_cast<cudaStream_t>(stream));
+}
+
 int pic_revolve_plan(int64_t n_steps, int64_t n_slots, int64_t *recompute_steps, int64_t *spine_levels) {
     return revolve_plan(n_steps, n_slots, recompute_steps, spine_levels);
 }

@@ -408,6 +408,8 @@ int revolve_backward(const pic_grid *g, void *slots_pos, void *slots_neg, int64_
                      void *adj_ws, cudaStream_t st);
 
 int selftest_waits(int32_t *barrier_status, int32_t *mbarrier_status, cudaStream_t st);
+int selftest_packets(const pic_grid *g, int32_t *step_status, int32_t *adjoint_status, int32_t *poisoned,
+                     cudaStream_t st);
 
 int sample_disc(const double *u, int64_t n_pairs, double scale, double mid, double radius_sq, int64_t n_wanted,
                 double *xs, double *ys, int64_t *n_accepted, int64_t *n_pairs_used);

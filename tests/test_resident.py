@@ -374,3 +374,32 @@ def test_derivative_sums_lose_no_bits(n, no_z, variant):
     want = steps * (scored.sum() * no_z - lam[0].sum())
     assert abs(want) < 2**44 and grad[4].item() == want
     assert np.array_equal(L[steps & 1].cpu().numpy(), lam[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,no_z,adjoint", [(24, 200, 7), (48, 200, 7), (76, 200, -1)])
+def test_packets_that_never_come_end_the_launch_with_a_status(n, no_z, adjoint):
+    """The resident kernels' bounded wait, with patches of one, two and six
+    columns: every block leaves, the status says why, the derivative sums are NaN,
+    and the context runs on."""
+    import torch
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    lib = native.load()
+    g = _grid(native, n, no_z, 0, native.PIC_F32, 0)
+    out = [ctypes.c_int32(-5) for _ in range(3)]
+    native.check(lib.pic_selftest_packets(ctypes.byref(g), *(ctypes.byref(o) for o in out),
+                                          torch.cuda.current_stream().cuda_stream), "pic_selftest_packets")
+    assert [o.value for o in out] == [7, adjoint, 1 if adjoint == 7 else 0]
+    state, xs, ys, off = _case(n, no_z, 9, n, 12)
+    got = _segment(native, g, torch, state, xs, ys, off, 0)
+    ref = _segment(native, _grid(native, n, no_z, 0, native.PIC_F64, 1), torch, state, xs, ys, off, 0)
+    _compare(native, got, ref, 9)
+
+
+def test_the_packet_selftest_needs_blocks_that_trade():
+    native = importlib.import_module(pkg().__name__ + "._native")
+    out = [ctypes.c_int32() for _ in range(3)]
+    for n, no_z in ((3, 1), (208, 400)):  # one block; not resident
+        g = _grid(native, n, no_z, 0, native.PIC_F32, 0)
+        assert native.load().pic_selftest_packets(ctypes.byref(g), *(ctypes.byref(o) for o in out), None) != native.PIC_OK
