@@ -229,9 +229,10 @@ class AdjointRun:
         # beyond the engine: lambda (two states) now or later, and the schedule's own
         seg_need = (self.n_seg + self.K) * state + n_dep * self.dslot * es
         avail = self._available(2 * state)
-        if self.schedule == "binomial" or seg_need > avail:
+        slots = min(self.slots_wanted or total, max(total, 1))
+        if (slots * state if self.schedule == "binomial" else seg_need) > avail:
             # the resident steps' and the deposition's part of the workspace is
-            # worth less than the room it takes (the binomial schedule has no use for it)
+            # worth less than the room it takes
             eng.use_step_workspace()
             avail = self._available(2 * state)
         kind = self.schedule
