@@ -30,10 +30,11 @@
 //   dR/dc+ += mu+[v] ((p~[v-z] - p~[v+z]) / 2 + c+ (p~[v-z] + p~[v+z] - 2 p~[v])),
 //   the same for the negative species with its z-swapped neighbours, and
 //   dR/da += [v scored] p~ n~ - (mu+[v] + mu-[v]) p~ n~.
-// The differences are formed per voxel before the products are summed: the
-// per-weight sums they combine are large and nearly equal, and subtracting
-// them after summation would cancel most of the float32 digits. The
-// deposition is a constant of every step: it enters only through u~.
+// The differences are formed per voxel before the products are summed (of u here;
+// of mu where the sums are taken by parts, as the eight-wide, the resident and the
+// streaming kernels do): the per-weight sums they combine are large and nearly
+// equal, and subtracting them after summation would cancel most of the float32
+// digits. The deposition is a constant of every step: it enters only through u~.
 //
 // lambda_s is written as zero on the z end planes (k = 0, nzb-1) and the row
 // padding: u there is fixed at zero whatever the parameters, so its adjoint
@@ -646,10 +647,14 @@ static int launch_adjoint_t(const pic_grid *g, const void *pos, const void *neg,
             return check_launch("wide_adjoint_kernel");
         }
     }
-    if (flat_index32(n, kp))
-        adjoint_step_kernel<T, BLOCK, uint32_t><<<(unsigned)blocks, BLOCK, 0, st>>>(a);
-    else
-        adjoint_step_kernel<T, BLOCK, int64_t><<<(unsigned)blocks, BLOCK, 0, st>>>(a);
+    // (float32: beyond 32-bit offsets)
+    if constexpr (sizeof(T) == 8) {
+        if (flat_index32(n, kp)) {
+            adjoint_step_kernel<T, BLOCK, uint32_t><<<(unsigned)blocks, BLOCK, 0, st>>>(a);
+            return check_launch("adjoint_step_kernel");
+        }
+    }
+    adjoint_step_kernel<T, BLOCK, int64_t><<<(unsigned)blocks, BLOCK, 0, st>>>(a);
     return check_launch("adjoint_step_kernel");
 }
 

@@ -101,16 +101,12 @@ __global__ void batched_prep_kernel(const pic_batch_cfg *cfgs, int n_cfgs, GridE
     table[c] = e;
 }
 
-
-// One entry of the work table (blk): a range of one grid's items, its
-// tallies reduced per block and (persistent form), by the grid's last block to
-// finish, into the grid's tally row; else left for batched_tallies_kernel. `red`, `last` and `a` are the caller's shared memory.
-template <typename T, int BLOCK, typename I, bool COH = false, bool WIDE = false>
-__device__ __forceinline__ void batched_step_block(const BatchStepArgs<T> &b, int blk,
-                                                   typename RedT<T>::type (*red)[4], bool &last, StepArgs<T> &a) {
-    using R = typename RedT<T>::type;
+// One entry of the work table (blk): a range of one grid's items and the
+// thread's share v of its tallies. `a` is the caller's shared memory.
+template <typename T, int BLOCK, typename I, bool COH, bool WIDE>
+__device__ __forceinline__ void batched_step_block(const BatchStepArgs<T> &b, int blk, typename RedT<T>::type (&v)[4],
+                                                   StepArgs<T> &a) {
     const int c = b.blk_cfg[blk];
-    const pic_batch_cfg &C = b.cfgs[c];
     if (threadIdx.x < 32) {  // one warp copies the grid's prepared arguments
         const GridEntry<T> *E = b.table + c;
         const uint32_t *src = reinterpret_cast<const uint32_t *>(&E->a);
@@ -127,7 +123,6 @@ __device__ __forceinline__ void batched_step_block(const BatchStepArgs<T> &b, in
         }
     }
     __syncthreads();
-    R v[4];
     bool stepped = false;
     if constexpr (WIDE) {
         const GridEntry<T> *E = b.table + c;
@@ -153,12 +148,17 @@ __device__ __forceinline__ void batched_step_block(const BatchStepArgs<T> &b, in
             flat_item<T, I, COH>(a, item, t_rec, t_p, t_n, t_inj);
         v[0] = red_of(t_inj), v[1] = red_of(t_rec), v[2] = red_of(t_p), v[3] = red_of(t_n);
     }
-    if constexpr (!COH) {
-        // the launches' tallies: batched_tallies_kernel, a group of steps at once
-        let_next_start();
-        leave_partial<BLOCK>(v, b.partials + 4 * (int64_t)blk);
-        return;
-    }
+}
+
+// The persistent form's tallies of an entry: reduced per block and, by the
+// grid's last block to finish, into the grid's tally row. `red`, `last` and `a`
+// are the caller's shared memory.
+template <typename T, int BLOCK>
+__device__ __forceinline__ void batched_finish_block(const BatchStepArgs<T> &b, int blk, typename RedT<T>::type (&v)[4],
+                                                     typename RedT<T>::type (*red)[4], bool &last, const StepArgs<T> &a) {
+    using R = typename RedT<T>::type;
+    const int c = b.blk_cfg[blk];
+    const pic_batch_cfg &C = b.cfgs[c];
     block_sum4<BLOCK>(v, red);
     if (threadIdx.x == 0) {
 #pragma unroll
@@ -196,13 +196,14 @@ __device__ __forceinline__ void batched_step_block(const BatchStepArgs<T> &b, in
 // and two waves of blocks 187 / 86 / 26.
 template <typename T, int BLOCK, typename I>
 __global__ void __launch_bounds__(BLOCK, sizeof(T) == 4 ? 4 : 1) batched_step_kernel(BatchStepArgs<T> b) {
-    __shared__ typename RedT<T>::type red[BLOCK / 32][4];
-    __shared__ bool last;
     // the block's grid arguments, staged once in shared memory and read by
     // broadcast (keeps them out of the registers of every thread)
     __shared__ StepArgs<T> a;
     wait_for_prev();
-    batched_step_block<T, BLOCK, I, false, sizeof(T) == 4 && sizeof(I) == 4>(b, blockIdx.x, red, last, a);
+    typename RedT<T>::type v[4];
+    batched_step_block<T, BLOCK, I, false, sizeof(T) == 4 && sizeof(I) == 4>(b, blockIdx.x, v, a);
+    let_next_start();
+    leave_partial<BLOCK>(v, b.partials + 4 * (int64_t)blockIdx.x);
 }
 
 // The tally rows of blockIdx.y consecutive steps of every grid of the work table
@@ -369,7 +370,9 @@ __global__ void __launch_bounds__(256) batched_persistent_kernel(BatchPersistArg
         b.step = s;
         for (int vb = blockIdx.x; vb < p.n_blocks; vb += gridDim.x) {
             __syncthreads();  // shared staging of the previous entry is done with
-            batched_step_block<T, BLOCK, I, true>(b, vb, red, last, a);
+            typename RedT<T>::type v[4];
+            batched_step_block<T, BLOCK, I, true, false>(b, vb, v, a);
+            batched_finish_block<T, BLOCK>(b, vb, v, red, last, a);
         }
         if (!grid_barrier(barrier_ref(p.bar))) return;
     }
@@ -439,12 +442,12 @@ int batched_status(const BatchLaunch &L, cudaStream_t st, int32_t *status) {
 }
 
 template <typename T, typename I>
-static void launch_batched_step(const BatchLaunch &L, int bi, int bo, double *partials, unsigned int *counters,
-                                int64_t step, cudaStream_t st, const void *dens, void *dens_zero) {
+static void launch_batched_step(const BatchLaunch &L, int bi, int bo, double *partials, int64_t step,
+                                cudaStream_t st, const void *dens, void *dens_zero) {
     constexpr int BLOCK = sizeof(T) == 4 && sizeof(I) == 4 ? 128 : 256;
     BatchStepArgs<T> b{L.cfgs, table_of<T>(L), L.blk_cfg, L.blk_item0, L.blk_item1, L.cfg_blk0, L.cfg_nblk,
                        (const T *)L.pos[bi], (const T *)L.neg[bi], (T *)L.pos[bo], (T *)L.neg[bo],
-                       (const pair_t<T> *)dens, (pair_t<T> *)dens_zero, L.tally, partials, counters, step,
+                       (const pair_t<T> *)dens, (pair_t<T> *)dens_zero, L.tally, partials, nullptr, step,
                        (((uintptr_t)L.pos[0] | (uintptr_t)L.pos[1] | (uintptr_t)L.neg[0] | (uintptr_t)L.neg[1]) & 31) == 0};
     launch_linked(batched_step_kernel<T, BLOCK, I>, (unsigned)L.n_blocks, BLOCK, st, b);
 }
@@ -603,7 +606,6 @@ static int batched_binned_deposit(const BatchLaunch &L, int64_t s0, int64_t s1, 
 int batched_loop(const BatchLaunch &L, cudaStream_t st) { return batched_loop_stream(L, nullptr, st); }
 
 int batched_loop_stream(const BatchLaunch &L, const pic_batch_stream *B, cudaStream_t st) {
-    unsigned int *counters = B ? nullptr : reinterpret_cast<unsigned int *>(L.workspace);
     if (L.n_steps > 0 && !B) {
         int rc = L.dtype == PIC_F64 ? prep_table<double>(L, st) : prep_table<float>(L, st);
         if (rc) return rc;
@@ -630,11 +632,11 @@ int batched_loop_stream(const BatchLaunch &L, const pic_batch_stream *B, cudaStr
         double *partials = partials_of(L) + 4 * (int64_t)L.n_blocks * waiting++;
         next = step + 1;
         if (L.dtype == PIC_F64) {
-            if (L.index32) launch_batched_step<double, uint32_t>(L, bi, bo, partials, counters, step, st, dens, dens_zero);
-            else launch_batched_step<double, int64_t>(L, bi, bo, partials, counters, step, st, dens, dens_zero);
+            if (L.index32) launch_batched_step<double, uint32_t>(L, bi, bo, partials, step, st, dens, dens_zero);
+            else launch_batched_step<double, int64_t>(L, bi, bo, partials, step, st, dens, dens_zero);
         } else {
-            if (L.index32) launch_batched_step<float, uint32_t>(L, bi, bo, partials, counters, step, st, dens, dens_zero);
-            else launch_batched_step<float, int64_t>(L, bi, bo, partials, counters, step, st, dens, dens_zero);
+            if (L.index32) launch_batched_step<float, uint32_t>(L, bi, bo, partials, step, st, dens, dens_zero);
+            else launch_batched_step<float, int64_t>(L, bi, bo, partials, step, st, dens, dens_zero);
         }
         return check_launch("batched_step_kernel");
     };

@@ -1,8 +1,8 @@
 // pic_wide.cuh -- the float32 body of the flat fused step: eight consecutive
 // k of one column a thread and pass, shared by the single-grid kernel
 // (step.cu) and the batched multi-grid kernel (batched.cu). Semantics as
-// flat_item (pic_flat.cuh), which float64 fields, grids beyond 32-bit
-// offsets, pointers without 32-byte alignment and the persistent kernels use.
+// flat_item (pic_flat.cuh), which float64 fields, grids beyond 32-bit offsets,
+// batched grids whose rows are not 32-byte aligned and the persistent kernels use.
 //
 // Why eight: decoding an item, its masks, offsets, scoring test and tallies
 // cost as much as its stencil, so the four-wide item took 305 instructions for

@@ -141,9 +141,15 @@ static int64_t flat_blocks(const pic_grid *g, bool wide, bool finish, bool run) 
 
 template <typename T, int BLOCK>
 static int launch_four_wide(const pic_grid *g, unsigned blocks, const StepArgs<T> &a, cudaStream_t st) {
-    // (items + stride stays below 2^32 on the 32-bit path: items < 2^29)
-    if (flat_index32(g->no_xy, g->kpitch)) launch_linked(step_kernel<T, BLOCK, uint32_t>, blocks, BLOCK, st, a);
-    else launch_linked(step_kernel<T, BLOCK, int64_t>, blocks, BLOCK, st, a);
+    // (items + stride stays below 2^32 on the 32-bit path: items < 2^29; float32
+    // grids come here beyond 32-bit offsets only)
+    if constexpr (sizeof(T) == 8) {
+        if (flat_index32(g->no_xy, g->kpitch)) {
+            launch_linked(step_kernel<T, BLOCK, uint32_t>, blocks, BLOCK, st, a);
+            return check_launch("step_kernel");
+        }
+    }
+    launch_linked(step_kernel<T, BLOCK, int64_t>, blocks, BLOCK, st, a);
     return check_launch("step_kernel");
 }
 
@@ -244,7 +250,7 @@ int StepRun::step(const void *pos_in, const void *neg_in, void *pos_out, void *n
 int step_occupancy(int dtype, int *blocks_per_sm) {
     cudaError_t e = dtype == PIC_F64
                         ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel<double, kFlatBlock<double>, uint32_t>, kFlatBlock<double>, 0)
-                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel<float, 256, uint32_t>, 256, 0);
+                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, step_kernel<float, 256, int64_t>, 256, 0);
     return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaOccupancyMaxActiveBlocksPerMultiprocessor", e);
 }
 
