@@ -147,18 +147,21 @@ int pic_step_workspace_bytes(const pic_grid *g, int64_t *bytes);
 
 /* Bytes of the workspace with which segments of this grid (pic_run_segment,
  * pic_graph_create, the gradient passes) run as the library prefers: the
- * step workspace and, for a float32 grid whose fields fit the SMs' registers
- * and shared memory (up to about a million cells), the resident step's part -- the
- * deposition pairs and track lists of 256 steps, the packets its blocks
- * exchange and their tally partials (20 to 200 MB). Allocated and passed as
- * the step workspace is; a workspace without that part is accepted and those
- * segments then run one launch a step. */
+ * step workspace and, for a grid of few 62 x 62-cell tiles, track lists and
+ * deposition pairs of as many steps as give every SM a few blocks (up to 256; a
+ * few MB to 50), or, for a float32 grid whose fields fit the SMs' registers and
+ * shared memory (up to about 1.7 million cells), the resident step's part -- those of
+ * 256 steps, the packets its blocks exchange and their tally partials (20 to 180
+ * MB). Allocated and passed as the step workspace is; a workspace without that
+ * part is accepted: segments then run one launch a step and deposit 8 steps at a
+ * time. */
 int pic_segment_workspace_bytes(const pic_grid *g, int64_t *bytes);
 
 /* 1 if segments of this grid run resident with such a workspace: its blocks
  * keep the fields on the chip for up to 256 steps a launch. That is the
- * library's choice for float32 grids of up to about a million cells with
- * variant AUTO, steps_per_launch 0, a deposit_variant other than TRACKS and
+ * library's choice for float32 grids that fit (up to about 1.7 million cells), and
+ * whose division over the SMs is estimated no slower than the flat step (few and
+ * tall columns, 51 x 51 x 606, are not), with variant AUTO, steps_per_launch 0, a deposit_variant other than TRACKS and
  * cutoff_voxels < 31.5 (segments of at least 4 steps, 65536 tracks a step at
  * most, none so dense that depositing step by step is faster); else 0. A segment of a few launches gains nothing from a CUDA graph. */
 int pic_segment_resident(const pic_grid *g, int32_t *resident);

@@ -38,11 +38,12 @@ from .pulses import TrackSampler, build_track_schedule
 from .state import Diagnostics, collection_efficiency
 
 # The batched step runs 4 resident blocks per SM (float32: 128 threads, 128
-# registers). Blocks are chosen per phase: WAVES per resident slot on phases of
+# registers; float64: 256 threads, 2 of them). Blocks are chosen per phase: WAVES per resident slot on phases of
 # at least SMALL_PHASE_ITEMS items, one per slot below: few, long blocks amortise
 # each block's set-up and reduction. Measured on a 32-configuration sweep (device
 # ms of the first 436 steps, 32 grids of 48.7 M cells), blocks per slot 1: 84.7,
-# 2: 83.2, 4: 86.0, 8: 90.7.
+# 2: 83.2, 4: 86.0, 8: 90.7. Float64 batches of 8 and 16 grids take 1.91 and 4.15 s
+# with 1, 2 or 4.
 BLOCKS_PER_SM = 4
 WAVES = 2
 WAVES_SMALL = 1

@@ -492,6 +492,11 @@ int launch_patch(const AdjResArgs &a, const ResPlan &p, cudaStream_t st) {
 
 }  // namespace
 
+// Taken wherever it fits. Measured, us a reverse step, resident / eight-wide, absorbing
+// wall: 10^2 x 56 4.3 / 6.0, 24^2 x 206 4.9 / 6.7, 48^2 x 206 8.2 / 9.5, 28^2 x 406 7.9 / 9.4,
+// 20^2 x 606 5.8 / 7.8; near its limits 56^2 x 206 12.5 / 11.1, 108^2 x 56 13.3 / 12.5;
+// reflecting (the other one folds the ring in a launch of its own) 4.4 / 8.1, 4.9 /
+// 8.6, 8.2 / 11.7, 8.0 / 11.4, 5.8 / 9.4, 11.0 / 12.8, 12.5 / 14.4.
 bool resident_adjoint_plan(const pic_grid *g, ResPlan *out) {
     static thread_local ResPlanMemo memo;
     return memo.plan(g, kAdjPatches, (int)(sizeof(kAdjPatches) / sizeof(kAdjPatches[0])), adj_smem, 1.7, out);
