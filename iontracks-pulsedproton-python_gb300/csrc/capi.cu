@@ -280,6 +280,9 @@ static int run_loop(const pic_grid *g, void *pos0, void *neg0, void *pos1, void 
         }
         return leave_pairs(g, dens, (int)((dens_parity + n_steps - 1) & 1), last_pairs, st);
     }
+    if (most > 0 && deposit_binned(g, ws, ws_bytes, -1)) {  // (steps of more than kBinTracks, in pieces)
+        if (int rc = clear_tile_counts(g, ws, st)) return rc;
+    }
     StepRun run(g, ws, n_steps, st);
     for (int64_t s = 0; s < n_steps; ++s) {
         const int bi = (int)((parity + s) & 1), bo = bi ^ 1;

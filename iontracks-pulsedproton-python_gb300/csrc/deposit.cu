@@ -255,12 +255,15 @@ AheadSpace ahead_space(const pic_grid *g) {
     return a;
 }
 
+int clear_tile_counts(const pic_grid *g, void *ws, cudaStream_t st) {
+    const cudaError_t e = cudaMemsetAsync(static_cast<char *>(ws) + kWorkspaceBytes, 0, (size_t)bin_count_bytes(g->no_xy), st);
+    return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaMemsetAsync(tile counts)", e);
+}
+
 int StepDeposits::begin() {
+    if (!space_.slots) return clear_tile_counts(g_, ws_, st_);
     const int64_t tiles = bin_tiles_per_side(g_->no_xy) * bin_tiles_per_side(g_->no_xy);
-    // (another grid may have left its own lists where this one's counts are)
-    const cudaError_t e = space_.slots
-        ? cudaMemsetAsync(static_cast<char *>(ws_) + space_.counts, 0, (size_t)(space_.slots * tiles * 4), st_)
-        : cudaMemsetAsync(static_cast<char *>(ws_) + kWorkspaceBytes, 0, (size_t)bin_count_bytes(g_->no_xy), st_);
+    const cudaError_t e = cudaMemsetAsync(static_cast<char *>(ws_) + space_.counts, 0, (size_t)(space_.slots * tiles * 4), st_);
     return e == cudaSuccess ? PIC_OK : set_cuda_error("cudaMemsetAsync(tile counts)", e);
 }
 

@@ -323,6 +323,10 @@ int launch_deposit_slots(const pic_grid *g, const double *xs, const double *ys, 
                          int64_t s1, uint32_t *hist, void *ws, int64_t counts, int64_t lists, void *dens,
                          int64_t dens_stride, int16_t *slot, cudaStream_t st);
 
+// Clears the tile counts of the step workspace before a segment: another grid
+// that shares it (a batch's grids that step alone) may have left its own lists
+// where this one's counts are.
+int clear_tile_counts(const pic_grid *g, void *ws, cudaStream_t st);
 // Of a step's `most` tracks, those a tile of the binned form meets on average.
 double bin_tile_tracks(const pic_grid *g, int64_t most);
 // Whether the deposition takes the binned form for this grid and workspace:

@@ -308,3 +308,47 @@ def test_the_gradients_forward_pass_deposits_in_groups_into_its_kept_slots(dtype
     ks_t, g_t, _ = A.ks_and_gradient(cfg, None, dtype=dtype, shape={"deposit_variant": "tracks"})
     assert ks_b == pytest.approx(ks_t, rel=tol)
     np.testing.assert_allclose(g_b, g_t, rtol=tol, atol=0)
+
+
+@pytest.mark.gpu
+def test_a_shared_workspace_keeps_no_counts_of_another_grid():
+    """Grids of a batch that step alone share one step workspace: a large grid's
+    step of more tracks than one launch pair takes, after a smaller grid has left
+    its track lists where the large one's tile counts are."""
+    import ctypes
+
+    import torch
+
+    from test_resident import _grid
+
+    native = importlib.import_module(pkg().__name__ + "._native")
+    lib = native.load()
+    rng = np.random.default_rng(4)
+    small, large = _grid(native, 300, 1, 0, native.PIC_F32, 1), _grid(native, 1055, 1, 0, native.PIC_F32, 1)
+    small.deposit_variant = native.PIC_DEPOSIT_BINNED
+    large.gaussian_factor = 1e-3
+    jobs = {300: (small, rng.uniform(2, 50, (2, 3000))), 1055: (large, rng.uniform(0, 1055, (2, 70000)))}
+
+    def run(order):
+        b = ctypes.c_int64()
+        native.check(lib.pic_segment_workspace_bytes(ctypes.byref(large), ctypes.byref(b)), "bytes")
+        ws = torch.zeros(b.value, dtype=torch.uint8, device="cuda")
+        for n in order:
+            g, xy = jobs[n]
+            f = [torch.zeros((n, n, g.kpitch), device="cuda") for _ in range(4)]
+            dens = [torch.zeros((n, 2 * ((n + 3) // 4 * 4)), device="cuda") for _ in range(2)]
+            counts = torch.zeros((n, n), dtype=torch.int32, device="cuda")
+            tally = torch.zeros((1, 4), dtype=torch.float64, device="cuda")
+            x, y = (torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in xy)
+            off = np.array([0, len(xy[0])], dtype=np.int64)
+            native.check(lib.pic_run_segment(
+                ctypes.byref(g), f[0].data_ptr(), f[1].data_ptr(), f[2].data_ptr(), f[3].data_ptr(), 0, 1, x.data_ptr(),
+                y.data_ptr(), off.ctypes.data, dens[0].data_ptr(), dens[1].data_ptr(), 0, counts.data_ptr(),
+                tally.data_ptr(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream), "pic_run_segment")
+        torch.cuda.synchronize()
+        return dens[0].cpu().numpy(), counts.cpu().numpy()
+
+    alone, after = run([1055]), run([300, 1055])
+    assert alone[1].sum() == 70000
+    for a, b in zip(alone, after):
+        assert np.array_equal(a, b)
